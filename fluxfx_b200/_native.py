@@ -75,6 +75,28 @@ class FfxGraphTail(C.Structure):
                 ('levels', FfxTailLevel * TAIL_LEVELS)]
 
 
+RELAX_LEVELS = 12
+
+
+class FfxRelaxGrid(C.Structure):
+    _fields_ = [('n', n3), ('inv', f3)]
+
+
+class FfxRelaxTile(C.Structure):
+    _fields_ = [('sweeps', i32), ('tile', n3)]
+
+
+class FfxRelaxLevel(C.Structure):
+    _fields_ = [('grid', FfxRelaxGrid), ('sweep', FfxRelaxTile), ('down', FfxRelaxTile), ('up', FfxRelaxTile),
+                ('p', vp), ('q', vp), ('rhs', vp)]
+
+
+class FfxRelaxPlan(C.Structure):
+    _fields_ = [('count', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32), ('tail', i32), ('tile', i32 * 2),
+                ('omega', f32), ('basis', vp), ('classes', vp), ('workspace_bytes', i64), ('workspace', vp),
+                ('level', FfxRelaxLevel * RELAX_LEVELS)]
+
+
 class FfxBrickStats(C.Structure):
     _fields_ = [("capacity", C.c_uint32), ("active", C.c_uint32), ("metadata_bytes", C.c_uint64)]
 
@@ -234,6 +256,10 @@ _PROTOTYPES = {
     'ffx_mg_prolong': (C.c_int, [n3, vp, vp, vp, vp]),
     'ffx_direct_solve': (C.c_int, [i32, vp, vp, f32, vp, vp]),
     'ffx_mg_residual_max': (C.c_int, [n3, f3, vp, vp, f32, vp, vp]),
+    'ffx_relax_plan': (C.c_int, [P(FfxRelaxPlan)]),
+    'ffx_relax_cycles': (C.c_int, [P(FfxRelaxPlan), i32, f32, i32, P(i32), vp]),
+    'ffx_relax_timeouts': (C.c_int, [P(FfxRelaxPlan), P(i32), vp]),
+    'ffx_relax_classes': (C.c_int, [n3, vp, vp, vp]),
     'ffx_graph_smooth': (C.c_int, [P(FfxGraphLevel), vp, vp, f32, vp, vp]),
     'ffx_graph_smooth2': (C.c_int, [P(FfxGraphLevel), vp, vp, f32, vp, vp, vp]),
     'ffx_graph_residual_max_smooth': (C.c_int, [P(FfxGraphLevel), vp, vp, f32, vp, vp, vp]),

@@ -107,11 +107,10 @@ class SolidPressureProjector(PressureProjector):
     def uses_impulse(self):
         return True
 
-    def solve_pressure(self, dt, previous_dt):
+    def _starts_from_zero(self, dt, previous_dt):
         # A short masked Jacobi solve cannot reliably remove a stale guess when
         # the new divergence is tiny: start from zero for stable damping.
-        self.pressure.zero_()
-        super().solve_pressure(dt, previous_dt)
+        return True
 
     def metrics(self):
         moving = self.settings.moving_colliders

@@ -16,6 +16,7 @@ from .. import _native as N
 from ..physics.config import validate_dt
 from ..physics.pressure import PressureSettings
 from .device import CudaDevice, KernelHandle, ptr, solids_struct
+from .relax import Relaxation
 
 
 class PressureProjector:
@@ -28,6 +29,8 @@ class PressureProjector:
         self._field_dtype = torch.bfloat16 if self.settings.storage == 'BF16' else torch.float32
         self._storage = N.FFX_F32 if self._field_dtype == torch.float32 else N.FFX_BF16
         self._mask = getattr(self.device, 'mask', None)
+        self._jacobi = None       # the Jacobi solve's plan (made on first use)
+        self._classes = None      # open-neighbour codes of the mask (ffx_relax_classes)
         self._solids = solids_struct(self.device)
         self.wall = KernelHandle('pressure_walls.glsl')
         self.divergence = KernelHandle('pressure_divergence.glsl')
@@ -225,18 +228,29 @@ class PressureProjector:
         gradient pass, or None: the pass then tests the mask itself."""
         return None
 
+    def _starts_from_zero(self, dt, previous_dt):
+        return previous_dt != dt
+
     def solve_pressure(self, dt, previous_dt):
-        if previous_dt != dt:
-            self.pressure.zero_()
         # Jacobi smooths across cells: scale the work with resolution squared.
         scaled = ceil(self.settings.pressure_iterations * max(1.0, (max(self.grid.shape) / 64) ** 2))
         multiplier = self.settings.pressure_cold_multiplier if previous_dt != dt else 1
         self.last_iterations = min(4096, scaled * multiplier)
-        omega = self.settings.pressure_relaxation
-        for _ in range(self.last_iterations):
-            self.device.call('ffx_jacobi', self._n3, self._inv3, self._mask_ptr(), ptr(self.pressure),
-                             ptr(self.before), dt, omega, ptr(self.spare), self.device.s)
-            self.pressure, self.spare = self.spare, self.pressure
+        if self._jacobi is None:
+            if self._mask is not None:
+                nx, ny, nz = self.grid.shape
+                with self.device.ordered():
+                    self._classes = torch.empty((nz, ny, (nx + 3) // 4 * 4), dtype=torch.uint8,
+                                                device=self.device.device)
+            self._jacobi = Relaxation(self.device, [self.grid.shape], self.grid.extent,
+                                      self.settings.pressure_relaxation, last=4096, classes=self._classes)
+        if self._classes is not None:
+            # the mask may have moved since the last solve
+            self.device.call('ffx_relax_classes', self._n3, self._mask_ptr(), ptr(self._classes), self.device.s)
+        self._jacobi.plan.last_sweeps = self.last_iterations
+        self._jacobi.plan.omega = self.settings.pressure_relaxation
+        self.pressure, self.spare = self._jacobi.run(self.pressure, self.spare, self.before, 1, dt,
+                                                     self._starts_from_zero(dt, previous_dt))
 
     # ------------------------------------------------------------- diagnostics
     def velocity_maxima(self):
@@ -286,4 +300,5 @@ class PressureProjector:
         self.ready = False
         self.last_dt = None
         self.bounded = None
+        self._jacobi = self._classes = None
         self.pressure = self.spare = self.before = self.after = None

@@ -42,6 +42,17 @@ def neumann_inverse(shape, extent):
     return _neumann_inverse_cached(tuple(int(n) for n in shape), tuple(float(e) for e in extent)).copy()
 
 
+def neumann_basis(shape, extent):
+    """The same inverse in separable form, one float64 vector: the cosine bases
+    of x, y and z (row-major, a row per mode), then 1 / eigenvalue of every mode
+    (x fastest; 0 for the constant mode)."""
+    (bx, ex), (by, ey), (bz, ez) = (_axis_basis(n, e) for n, e in zip(shape, extent))
+    lam = (ez[:, None, None] + ey[None, :, None] + ex[None, None, :]).ravel()
+    inv_lam = np.zeros_like(lam)
+    inv_lam[1:] = 1.0 / lam[1:]
+    return np.concatenate([bx.ravel(), by.ravel(), bz.ravel(), inv_lam])
+
+
 def coarse_inverse(extent):
     """The reference's 4^3 table: 4096 floats, row-major (row = output cell)."""
     return tuple(neumann_inverse((4, 4, 4), extent).ravel().tolist())

@@ -362,6 +362,58 @@ int ffx_direct_solve(int32_t n, const double* inverse, const float* rhs, float d
 int ffx_mg_residual_max(const int32_t n[3], const float inv[3], const float* p,
                         const float* rhs, float dt, float* out, void* stream);
 
+/* ------------------------------------------- relaxation, whole solves */
+/* The same weighted Jacobi sweeps and V-cycles (backend/multigrid.py:20-95,
+ * backend/pressure.py:57-98), whole solves at a time: one cooperative launch
+ * with the iterate resident on the chip where the grid fits (128^3 and less),
+ * else several sweeps per launch. Results equal the single passes' to FP32
+ * rounding. */
+#define FFX_RELAX_LEVELS 12
+typedef struct FfxRelaxGrid {
+    int32_t n[3];       /* cells, at least 2 per axis */
+    float inv[3];       /* 1 / spacing */
+} FfxRelaxGrid;
+typedef struct FfxRelaxTile {
+    int32_t sweeps;     /* sweeps of one launch */
+    int32_t tile[3];    /* cells a block writes */
+} FfxRelaxTile;
+typedef struct FfxRelaxLevel {
+    FfxRelaxGrid grid;
+    FfxRelaxTile sweep, down, up;   /* filled by ffx_relax_plan for grids that are not resident */
+    float* p;
+    float* q;           /* second iterate; p, q and rhs below level 0 only where the grid is not resident */
+    float* rhs;         /* level 0: the divergence; below: written by the cycles */
+} FfxRelaxLevel;
+typedef struct FfxRelaxPlan {
+    int32_t count, pre, post;
+    int32_t last_sweeps;  /* sweeps of the coarsest level without a direct solve */
+    int32_t tail;         /* filled: first level that one block holds whole */
+    int32_t tile[2];      /* filled: rows (y, z) of a resident tile; 0 when the grid is not resident */
+    float omega;
+    /* Direct solve of the coarsest level (at most 512 cells), or NULL: device
+     * FP64 cosine basis bx (nx x nx, a row per mode), by, bz, then 1 / eigenvalue
+     * of every mode (x fastest; 0 for the constant mode). */
+    const double* basis;
+    const uint8_t* classes;   /* one level only: ffx_relax_classes of a collider mask, or NULL */
+    int64_t workspace_bytes;  /* filled */
+    void* workspace;          /* caller's, 16-byte aligned, zeroed once; for one solve at a time */
+    FfxRelaxLevel level[FFX_RELAX_LEVELS];
+} FfxRelaxPlan;
+/* Fills the plan for its grids (host only). Whether classes is NULL matters here. */
+int ffx_relax_plan(FfxRelaxPlan* plan);
+/* `cycles` V-cycles on L p = rhs / dt; with one level, `cycles` times last_sweeps
+ * weighted Jacobi sweeps. from_zero: the iterate starts from zero and level 0's
+ * p is not read. *swapped = 1 when the result is in level 0's q. */
+int ffx_relax_cycles(const FfxRelaxPlan* plan, int32_t cycles, float dt, int32_t from_zero,
+                     int32_t* swapped, void* stream);
+/* Bounded waits of resident solves that gave up, since the workspace was zeroed
+ * (waits for the stream). Anything but 0 means wrong pressures. */
+int ffx_relax_timeouts(const FfxRelaxPlan* plan, int32_t* count, void* stream);
+/* One byte per cell: open neighbours cx + 3 cy + 9 cz along the axes, 27 in a
+ * solid; rows padded to a multiple of four bytes (with 27), so `classes` holds
+ * 4 ceil(nx / 4) * ny * nz bytes and starts on 4. */
+int ffx_relax_classes(const int32_t n[3], const uint8_t* solid, uint8_t* classes, void* stream);
+
 /* ------------------------------------- collider (aggregation) multigrid */
 /* A level of the graph Laplacian. Level 0 derives its conductances from the
  * solid mask (edges == NULL): w[a] between two fluid cells, 0 otherwise. Coarse
