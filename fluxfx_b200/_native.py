@@ -122,6 +122,13 @@ class FfxConv(C.Structure):
                 ('out_f32_pitch', i32)]
 
 
+ADAM_SLOTS = 64
+
+
+class FfxAdamSlot(C.Structure):
+    _fields_ = [('n', i64), ('w', vp), ('m', vp), ('v', vp), ('g', vp), ('w_bf16', vp)]
+
+
 BATCH_MAX = 64
 BATCH_LEVELS = 8
 (PASS_PREDICTOR, PASS_VELOCITY, PASS_DIVERGENCE, PASS_SCALE, PASS_GRADIENT, PASS_SCALAR_PREDICTOR,
@@ -285,6 +292,9 @@ _PROTOTYPES = {
     'ffx_bias_grad': (C.c_int, [i64, i32, vp, i32, vp, vp]),
     'ffx_weight_transpose': (C.c_int, [i32, i32, i32, i32, vp, vp, vp]),
     'ffx_adam': (C.c_int, [i64, vp, vp, vp, vp, vp, f32, f32, f32, f32, i32, vp]),
+    'ffx_adam_many': (C.c_int, [i32, P(FfxAdamSlot), f32, f32, f32, f32, i32, vp]),
+    'ffx_relu_bias_backward': (C.c_int, [i64, i32, vp, i32, vp, i32, i32, vp, vp]),
+    'ffx_mse_grad_masked': (C.c_int, [i64, vp, i32, vp, vp, vp, vp, vp, vp]),
     'ffx_pack_input': (C.c_int, [i64, vp, vp, f32, vp, vp]),
     'ffx_mse_grad': (C.c_int, [i64, vp, i32, vp, vp, f32, vp, vp, vp]),
     'ffx_unpack_channel': (C.c_int, [i64, vp, i32, f32, vp, vp]),

@@ -21,7 +21,9 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <type_traits>
 
 #include "ffx_host.cuh"
 
@@ -33,7 +35,6 @@ using bf16 = __nv_bfloat16;
 constexpr int kBM = 128, kBN = 64, kStages = 3, kGemmThreads = 128;
 constexpr int kAStride = 24;    // bf16 per A row in shared memory (16 + 8 pad: 48 B, conflict-free ldmatrix)
 constexpr int kBStride = 72;    // bf16 per B row (64 + 8 pad: 144 B)
-constexpr int kWStride = 136;   // bf16 per A row of the weight-gradient tile (128 + 8 pad: 272 B)
 
 struct View {
     const bf16* p;
@@ -75,6 +76,10 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned r[4], const void* sme
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(s));
+}
+__device__ __forceinline__ void ldmatrix_x2_trans(unsigned r[2], const void* smem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(s));
 }
 __device__ __forceinline__ void mma_bf16(float c[4], const unsigned a[4], unsigned b0, unsigned b1) {
     asm volatile(
@@ -880,93 +885,188 @@ __global__ void conv3_pack_kernel(const bf16* __restrict__ w, int cin, int cout,
 // ------------------------------------------------------ weight gradient GEMM
 // dW[k][n] += sum over the block's voxel chunk of A[m][k] G[m][n]; A^T
 // fragments come from the [m][k] tile through ldmatrix.trans.
-__global__ void __launch_bounds__(kGemmThreads) conv_wgrad_kernel(const __grid_constant__ Conv a, const bf16* g,
-                                                                 int g_pitch, float* dw, long long chunk) {
-    __shared__ __align__(128) bf16 sA[kStages][16 * kWStride];
-    __shared__ __align__(128) bf16 sG[kStages][16 * kBStride];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k0 = blockIdx.x * 128, n0 = blockIdx.y * kBN;
-    const int cls = a.transposed ? (int)(blockIdx.z % 8) : 0;
-    const long long split = a.transposed ? blockIdx.z / 8 : blockIdx.z;
-    const long long mb = split * chunk;
-    const long long me = min(a.rows, mb + chunk);
-    const int nsteps = (int)((me - mb + 15) / 16);
-    const int u0 = k0 / 8;
+//
+// What bounds it is the chain of MMAs into one accumulator: a chunk of 8192
+// voxels is 512 of them in a row, whatever the tile. So the tile is narrow (64
+// input by 16 or 32 output channels; a warp has 16 of the former and half of
+// the latter), a step is one or two MMAs long, and a layer of one chunk still
+// fills the SMs (64 -> 64 channels: 54 blocks). A stage is 64 voxels and up to
+// six are in flight, so a step never waits for its gathers, and a gather costs
+// a dozen instructions: its tap is fixed per thread and its voxel's position
+// moves by carries, not divisions. Every accumulator sums its voxels in the
+// order of the 16-voxel steps, so a chunk's sums do not depend on the tile.
+// With a 128 x 64 tile, three 16-voxel stages and 64-bit divisions per gather a
+// step took 1.4 us and a layer 730 us.
+constexpr int kWgVox = 64, kWgK = 64, kWgStages = 6, kWgThreads = 256;
 
-    auto load = [&](int stage, int step) {
-        const int ml = tid >> 3;
-        const long long m = mb + (long long)step * 16 + ml;
-        const bool row_ok = m < me;
-        RowPos pos = {0, 0, 0, 0};
-        if (row_ok) pos = a.transposed ? decode(m, a.id, a.ih, a.iw) : decode(m, a.od, a.oh, a.ow);
+struct Wgrad {
+    Conv a;
+    const bf16* g;
+    int g_pitch;
+    float* dw;
+    int chunk;
+    int w, h, d;               // the GEMM row's grid (output voxels, or input voxels per parity class)
+    int step_x, step_y, step_z;   // kWgVox rows further, in that grid
+};
+
+// Position of a GEMM row that moves on by kWgVox rows at a time.
+struct Walk {
+    int x, y, z, b;
+    __device__ __forceinline__ void start(const Wgrad& P, int m) {
+        const int r = m / P.w, t = r / P.h;
+        x = m - r * P.w;
+        y = r - t * P.h;
+        b = t / P.d;
+        z = t - b * P.d;
+    }
+    __device__ __forceinline__ void advance(const Wgrad& P) {
+        x += P.step_x;
+        y += P.step_y;
+        z += P.step_z;
+        if (x >= P.w) { x -= P.w; ++y; }
+        if (y >= P.h) { y -= P.h; ++z; }
+        while (z >= P.d) { z -= P.d; ++b; }
+    }
+};
+
+// How a GEMM row's input voxel follows from it: the same voxel shifted by the
+// tap (padded stride-1 convolutions: the address moves on by a constant), the
+// strided convolution's, or the row itself (transposed: the gradient's voxel
+// is the strided one).
+enum WgKind { kWgSame = 0, kWgStrided = 1, kWgTransposed = 2 };
+
+template <int NT, int KIND>
+__global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(const __grid_constant__ Wgrad P) {
+    constexpr int AS = kWgK + 8, GS = NT + 8;      // bf16 per shared row (8 pad: conflict-free ldmatrix)
+    constexpr int NW = NT / 2;                     // output channels of a warp
+    constexpr int kRows = kWgThreads / 8;          // voxels that the block's gathers cover at once
+    extern __shared__ __align__(128) unsigned char wg_smem[];
+    bf16* sA = reinterpret_cast<bf16*>(wg_smem);
+    bf16* sG = sA + kWgStages * kWgVox * AS;
+    const Conv& a = P.a;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int k0 = blockIdx.x * kWgK, n0 = blockIdx.y * NT;
+    const int cls = KIND == kWgTransposed ? (int)(blockIdx.z % 8) : 0;
+    const int split = KIND == kWgTransposed ? (int)(blockIdx.z / 8) : (int)blockIdx.z;
+    const int mb = split * P.chunk;
+    const int rows = (int)min(a.rows - mb, (long long)P.chunk);
+    const int stages = (rows + kWgVox - 1) / kWgVox;
+
+    // this thread's input channels (one unit of 8 at one tap) for every voxel it gathers
+    const int u = k0 / 8 + (tid & 7);
+    const bool unit_ok = u < a.k_units;
+    const int tap = KIND == kWgTransposed ? 0 : u / a.units_per_tap;
+    const int c = (u - tap * a.units_per_tap) * 8;
+    const int dz = tap / (a.ks * a.ks) - a.pad, dy = tap / a.ks % a.ks - a.pad, dx = tap % a.ks - a.pad;
+    const bool second = c >= a.c1;
+    const bf16* in = second ? a.in2.p + a.in2.offset + (c - a.c1) : a.in1.p + a.in1.offset + c;
+    const int pitch = second ? a.in2.pitch : a.in1.pitch;
+    // and its gradient channels
+    constexpr int kUnits = NT / 8;
+    const int g_row = tid / kUnits, g_ch = tid % kUnits * 8;
+    const bool g_ok = g_row < kWgVox && n0 + g_ch < a.cout;
+    constexpr int kMine = kWgVox / kRows;
+    Walk walk[kMine], g_walk;
+    const bf16* src[kMine];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int ul = (tid & 7) * 2 + h;
-            const int u = u0 + ul;
-            const bf16* src = (row_ok && u < a.k_units) ? gather(a, pos, u) : nullptr;
-            cp_async16(&sA[stage][ml * kWStride + ul * 8], src ? src : a.in1.p, src != nullptr);
+    for (int i = 0; i < kMine; ++i) {
+        const int m = mb + (tid >> 3) + kRows * i;
+        walk[i].start(P, m);
+        src[i] = in + (m + (KIND == kWgSame ? (dz * P.h + dy) * P.w + dx : 0)) * (long long)pitch;
+    }
+    g_walk.start(P, mb + g_row);
+    const bf16* g_src = P.g + (mb + g_row) * (long long)P.g_pitch + n0 + g_ch;
+
+    int left = rows - (tid >> 3), g_left = rows - g_row;     // rows from this thread's on, at the next stage
+    auto load = [&](int slot) {         // stages in order: the walks and addresses move on
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
+            bool ok = unit_ok && left > kRows * i;
+            const bf16* from = src[i];
+            if (KIND == kWgSame) {
+                ok = ok && (unsigned)(walk[i].x + dx) < (unsigned)P.w && (unsigned)(walk[i].y + dy) < (unsigned)P.h &&
+                     (unsigned)(walk[i].z + dz) < (unsigned)P.d;
+            } else if (KIND == kWgStrided) {
+                const int xx = walk[i].x * a.stride + dx, yy = walk[i].y * a.stride + dy,
+                          zz = walk[i].z * a.stride + dz;
+                ok = ok && (unsigned)zz < (unsigned)a.id && (unsigned)yy < (unsigned)a.ih &&
+                     (unsigned)xx < (unsigned)a.iw;
+                from = in + ((((long long)walk[i].b * a.id + zz) * a.ih + yy) * a.iw + xx) * pitch;
+            }
+            cp_async16(sA + (slot * kWgVox + (tid >> 3) + kRows * i) * AS + (tid & 7) * 8, ok ? from : a.in1.p, ok);
+            if (KIND != kWgTransposed) walk[i].advance(P);
+            src[i] += (long long)kWgVox * pitch;
         }
-        const int nu = (tid & 7) * 8, n = n0 + nu;
-        const bool ok = row_ok && n < a.cout;
-        const bf16* src = ok ? g + out_voxel(a, m, cls) * g_pitch + n : g;
-        cp_async16(&sG[stage][ml * kBStride + nu], src, ok);
+        if (g_row < kWgVox) {
+            const bool ok = g_ok && g_left > 0;
+            const bf16* from = g_src;
+            if (KIND == kWgTransposed) {
+                from = P.g + n0 + g_ch + ((((long long)g_walk.b * a.od + 2 * g_walk.z + (cls >> 2)) * a.oh +
+                                           2 * g_walk.y + (cls >> 1 & 1)) * a.ow + 2 * g_walk.x + (cls & 1)) * P.g_pitch;
+                g_walk.advance(P);
+            }
+            cp_async16(sG + (slot * kWgVox + g_row) * GS + g_ch, ok ? from : P.g, ok);
+            g_src += (long long)kWgVox * P.g_pitch;
+        }
+        left -= kWgVox;
+        g_left -= kWgVox;
     };
 
-    float acc[2][8][4];
+    float acc[NW / 8][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < NW / 8; ++j)
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+        for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
 
+    const int kw = (warp & 3) * 16, nw = (warp >> 2) * NW;
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
-        if (s < nsteps) load(s, s);
+    for (int s = 0; s < kWgStages - 1; ++s) {
+        if (s < stages) load(s);
         cp_async_commit();
     }
-    for (int step = 0; step < nsteps; ++step) {
-        cp_async_wait<kStages - 2>();
+    int slot = 0, fill = kWgStages - 1;
+    for (int s = 0; s < stages; ++s) {
+        cp_async_wait<kWgStages - 2>();
         __syncthreads();
-        const int pf = step + kStages - 1;
-        if (pf < nsteps) load(pf % kStages, pf);
+        if (s + kWgStages - 1 < stages) load(fill);
         cp_async_commit();
-        const int st = step % kStages;
-        unsigned af[2][4];
+        const bf16* A = sA + slot * kWgVox * AS + ((lane & 7) + ((lane >> 4) << 3)) * AS + kw + ((lane >> 3) & 1) * 8;
+        const bf16* G = sG + slot * kWgVox * GS + ((lane & 7) + ((lane >> 3) & 1) * 8) * GS + nw +
+                        (NW == 16 ? (lane >> 4) * 8 : 0);
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const int kt = warp * 2 + mt;
-            ldmatrix_x4_trans(af[mt], &sA[st][((lane & 7) + ((lane >> 4) << 3)) * kWStride + kt * 16 +
-                                              ((lane >> 3) & 1) * 8]);
-        }
-#pragma unroll
-        for (int np = 0; np < 4; ++np) {
-            unsigned bf[4];
-            ldmatrix_x4_trans(bf, &sG[st][((lane & 7) + ((lane >> 3) & 1) * 8) * kBStride + np * 16 + (lane >> 4) * 8]);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                mma_bf16(acc[mt][2 * np], af[mt], bf[0], bf[1]);
-                mma_bf16(acc[mt][2 * np + 1], af[mt], bf[2], bf[3]);
+        for (int step = 0; step < kWgVox / 16; ++step) {
+            // (rows past the chunk's end were staged as zeros and add nothing)
+            unsigned af[4];
+            ldmatrix_x4_trans(af, A + 16 * step * AS);
+            if (NW == 16) {
+                unsigned bf[4];
+                ldmatrix_x4_trans(bf, G + 16 * step * GS);
+                mma_bf16(acc[0], af, bf[0], bf[1]);
+                mma_bf16(acc[NW / 8 - 1], af, bf[2], bf[3]);
+            } else {
+                unsigned bf[2];
+                ldmatrix_x2_trans(bf, G + 16 * step * GS);
+                mma_bf16(acc[0], af, bf[0], bf[1]);
             }
         }
+        slot = slot + 1 == kWgStages ? 0 : slot + 1;
+        fill = fill + 1 == kWgStages ? 0 : fill + 1;
     }
     cp_async_wait<0>();
     const int k_elems = a.k_units * 8;
-    float* base = dw + (a.transposed ? (size_t)cls * a.cin * a.cout : 0);
+    float* base = P.dw + (size_t)cls * a.cin * a.cout;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int half = 0; half < 2; ++half) {
+        const int k = k0 + kw + (lane >> 2) + half * 8;
+        if (k >= k_elems) continue;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int k = k0 + warp * 32 + mt * 16 + (lane >> 2) + half * 8;
-            if (k >= k_elems) continue;
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                const int n = n0 + nt * 8 + (lane & 3) * 2;
-                if (n >= a.cout) continue;
-                atomicAdd(base + (size_t)k * a.cout + n, acc[mt][nt][half * 2]);
-                atomicAdd(base + (size_t)k * a.cout + n + 1, acc[mt][nt][half * 2 + 1]);
-            }
+        for (int nt = 0; nt < NW / 8; ++nt) {
+            const int n = n0 + nw + nt * 8 + (lane & 3) * 2;
+            if (n >= a.cout) continue;
+            atomicAdd(base + (size_t)k * a.cout + n, acc[nt][half * 2]);
+            atomicAdd(base + (size_t)k * a.cout + n + 1, acc[nt][half * 2 + 1]);
         }
+    }
 }
 
 // ------------------------------------------------------------ elementwise
@@ -978,6 +1078,46 @@ __global__ void relu_backward_kernel(long long voxels, int channels, bf16* dy, i
     const long long v = i / channels;
     const int c = (int)(i - v * channels);
     if (!(__bfloat162float(y[v * y_pitch + y_offset + c]) > 0.f)) dy[v * dy_pitch + c] = __float2bfloat16_rn(0.f);
+}
+
+// The ReLU derivative of a layer's output gradient, in place, and its bias
+// gradient, in one pass over 16-byte groups of 8 channels (a separate scalar
+// pass each took 29 + 11 us at 64^3 x 2 x 16 channels; the bytes take 8). A
+// thread keeps one group of channels; blocks end with one atomic per channel.
+__global__ void __launch_bounds__(256) relu_bias_kernel(long long voxels, int channels, bf16* dy, int dy_pitch,
+                                                        const bf16* __restrict__ y, int y_pitch, int y_offset,
+                                                        float* db) {
+    __shared__ float part[128];
+    const int groups = channels / 8, c = threadIdx.x % groups * 8;
+    for (int i = threadIdx.x; i < channels; i += blockDim.x) part[i] = 0.f;
+    __syncthreads();
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const int rows = blockDim.x / groups;
+    for (long long v = (long long)blockIdx.x * rows + threadIdx.x / groups; v < voxels;
+         v += (long long)gridDim.x * rows) {
+        uint4* at = reinterpret_cast<uint4*>(dy + v * dy_pitch + c);
+        uint4 g = *at;
+        bf16* h = reinterpret_cast<bf16*>(&g);
+        if (y) {
+            const uint4 o = __ldg(reinterpret_cast<const uint4*>(y + v * y_pitch + y_offset + c));
+            const bf16* k = reinterpret_cast<const bf16*>(&o);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (!(__bfloat162float(k[e]) > 0.f)) h[e] = __float2bfloat16_rn(0.f);
+            *at = g;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum[e] += __bfloat162float(h[e]);
+    }
+    // lanes of a warp with the same channels (groups is a power of two up to 16)
+    for (int o = groups; o < 32; o <<= 1)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
+    if ((threadIdx.x & 31) < groups)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) atomicAdd(&part[c + e], sum[e]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < channels; i += blockDim.x) atomicAdd(db + i, part[i]);
 }
 
 // db[c] += sum over voxels of g[v][c] (block-local FP32 sums, one atomic per channel and block).
@@ -1016,6 +1156,27 @@ __global__ void adam_kernel(long long n, float* w, float* m, float* v, const flo
 // channels 2..7 = 0 (the first convolution reads 8 channels).
 // out = src * scale; with `max_abs`, scale = 1 / (input_scale * weight) in
 // FP64 (0 for a zero input), the factor that undoes the input normalisation.
+// adam_kernel for all parameter tensors of a network in one launch (blockIdx.y:
+// the tensor): 42 launches of 3 us each were latency only.
+struct AdamMany {
+    FfxAdamSlot slot[FFX_ADAM_SLOTS];
+    float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(256) adam_many_kernel(const __grid_constant__ AdamMany P) {
+    const FfxAdamSlot& s = P.slot[blockIdx.y];
+    bf16* w16 = (bf16*)s.w_bf16;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += (long long)gridDim.x * blockDim.x) {
+        const float gi = s.g[i];
+        const float mi = P.b1 * s.m[i] + (1.f - P.b1) * gi;
+        const float vi = P.b2 * s.v[i] + (1.f - P.b2) * gi * gi;
+        s.m[i] = mi;
+        s.v[i] = vi;
+        const float wi = s.w[i] - P.lr * (mi / P.c1) / (sqrtf(vi / P.c2) + P.eps);
+        s.w[i] = wi;
+        if (w16) w16[i] = __float2bfloat16_rn(wi);
+    }
+}
+
 __global__ void unpack_channel_kernel(long long voxels, const float* __restrict__ src, int pitch, float scale,
                                       const float* max_abs, double weight, float* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1066,14 +1227,17 @@ __global__ void pack_input_kernel(long long voxels, const float* div, const uint
 // Loss sum_v (pred - target)^2 / count over fluid voxels and its gradient,
 // written into channel 0 of an 8-channel BF16 tensor (the head's input gradient
 // is formed from it by the head's data-gradient convolution).
+// `fluid`: the count of fluid voxels on the device (fluid_count_kernel), for
+// 1 / max(count, 1), or NULL for inv_count.
 __global__ void mse_kernel(long long voxels, const float* pred, int pred_pitch, const float* target,
-                           const uint8_t* mask, float inv_count, bf16* grad, double* loss) {
-    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+                           const uint8_t* mask, float inv_count, const int* fluid, bf16* grad, double* loss) {
+    if (fluid) inv_count = (float)(1.0 / (double)max(*fluid, 1));
     double e = 0.0;
-    if (v < voxels) {
-        const bool fluid = !(mask && mask[v]);
-        const float d = fluid ? pred[v * pred_pitch] - target[v] : 0.f;
-        e = (double)d * d * inv_count;
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < voxels;
+         v += (long long)gridDim.x * blockDim.x) {
+        const bool open = !(mask && mask[v]);
+        const float d = open ? pred[v * pred_pitch] - target[v] : 0.f;
+        e += (double)d * d * inv_count;
         __align__(16) bf16 c[8];
         c[0] = __float2bfloat16_rn(2.f * d * inv_count);
 #pragma unroll
@@ -1082,6 +1246,16 @@ __global__ void mse_kernel(long long voxels, const float* pred, int pred_pitch, 
     }
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
     if ((threadIdx.x & 31) == 0 && e != 0.0) atomicAdd(loss, e);
+}
+
+// *count += voxels - sum of the mask (its fluid voxels where it holds 0 and 1).
+__global__ void fluid_count_kernel(long long voxels, const uint8_t* __restrict__ mask, int* count) {
+    int n = 0;
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < voxels;
+         v += (long long)gridDim.x * blockDim.x)
+        n += 1 - (int)mask[v];
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
 }
 
 // dst[t][co][ci] = src[flip ? taps - 1 - t : t][ci][co]: the weights of the
@@ -1375,11 +1549,46 @@ int ffx_conv_weight_grad(const FfxConv* c, const void* grad, int32_t grad_pitch,
                 "ffx_conv_weight_grad: invalid gradient view");
     const long long chunk = 8192;
     const long long splits = (a.rows + chunk - 1) / chunk;
-    FFX_REQUIRE(splits * (a.transposed ? 8 : 1) < 65536, "ffx_conv_weight_grad: too many voxels for one launch");
-    const dim3 grid((unsigned)((a.k_units * 8 + 127) / 128), (unsigned)((a.cout + kBN - 1) / kBN),
-                    (unsigned)(splits * (a.transposed ? 8 : 1)));
-    conv_wgrad_kernel<<<grid, kGemmThreads, 0, as_stream(stream)>>>(a, (const bf16*)grad, grad_pitch, dweight, chunk);
-    return launch_status("conv_wgrad_kernel");
+    FFX_REQUIRE(splits * (a.transposed ? 8 : 1) < 65536 && a.rows < (1ll << 31),
+                "ffx_conv_weight_grad: too many voxels for one launch");
+    Wgrad P = {};
+    P.a = a;
+    P.g = (const bf16*)grad;
+    P.g_pitch = grad_pitch;
+    P.dw = dweight;
+    P.chunk = (int)chunk;
+    P.w = a.transposed ? a.iw : a.ow;
+    P.h = a.transposed ? a.ih : a.oh;
+    P.d = a.transposed ? a.id : a.od;
+    P.step_x = kWgVox % P.w;
+    P.step_y = kWgVox / P.w % P.h;
+    P.step_z = kWgVox / P.w / P.h;
+    // 16 output channels a block where the layer has no more, else 32
+    auto launch = [&](auto nt, auto kind) {
+        constexpr int NT = decltype(nt)::value, KIND = decltype(kind)::value;
+        constexpr int smem = kWgStages * kWgVox * (kWgK + 8 + NT + 8) * (int)sizeof(bf16);
+        static std::atomic<uint64_t> ready{0};
+        int dev = 0;
+        cudaError_t err = cudaGetDevice(&dev);
+        if (err == cudaSuccess && !(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
+            err = cudaFuncSetAttribute(conv_wgrad_kernel<NT, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (err == cudaSuccess) ready.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_release);
+        }
+        if (err != cudaSuccess) return cuda_status(err, "ffx_conv_weight_grad");
+        const dim3 grid((unsigned)((a.k_units * 8 + kWgK - 1) / kWgK), (unsigned)((a.cout + NT - 1) / NT),
+                        (unsigned)(splits * (a.transposed ? 8 : 1)));
+        conv_wgrad_kernel<NT, KIND><<<grid, kWgThreads, smem, as_stream(stream)>>>(P);
+        return launch_status("conv_wgrad_kernel");
+    };
+    const std::integral_constant<int, kWgSame> same;
+    const std::integral_constant<int, kWgStrided> strided;
+    const std::integral_constant<int, kWgTransposed> transposed;
+    const std::integral_constant<int, 16> narrow;
+    const std::integral_constant<int, 32> wide;
+    if (a.transposed) return a.cout <= 16 ? launch(narrow, transposed) : launch(wide, transposed);
+    if (a.stride == 1 && a.id == a.od && a.ih == a.oh && a.iw == a.ow)
+        return a.cout <= 16 ? launch(narrow, same) : launch(wide, same);
+    return a.cout <= 16 ? launch(narrow, strided) : launch(wide, strided);
 }
 
 int ffx_relu_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pitch, const void* y, int32_t y_pitch,
@@ -1408,6 +1617,43 @@ int ffx_adam(int64_t n, float* w, float* m, float* v, const float* g, void* w_bf
     adam_kernel<<<blocks_for(n, 256), 256, 0, as_stream(stream)>>>(n, w, m, v, g, (bf16*)w_bf16, lr, beta1, beta2,
                                                                     eps, c1, c2);
     return launch_status("adam_kernel");
+}
+
+int ffx_adam_many(int32_t count, const FfxAdamSlot* slots, float lr, float beta1, float beta2, float eps, int32_t step,
+                  void* stream) {
+    FFX_REQUIRE(count >= 1 && count <= FFX_ADAM_SLOTS && slots && step >= 1 && lr > 0.f,
+                "ffx_adam_many: invalid arguments");
+    AdamMany P;
+    int64_t most = 1;
+    for (int k = 0; k < count; ++k) {
+        const FfxAdamSlot& s = slots[k];
+        FFX_REQUIRE(s.n >= 1 && s.w && s.m && s.v && s.g, "ffx_adam_many: slot %d is incomplete", k);
+        P.slot[k] = s;
+        most = std::max<int64_t>(most, s.n);
+    }
+    P.lr = lr;
+    P.b1 = beta1;
+    P.b2 = beta2;
+    P.eps = eps;
+    P.c1 = 1.f - powf(beta1, (float)step);
+    P.c2 = 1.f - powf(beta2, (float)step);
+    const dim3 grid((unsigned)std::min<int64_t>(blocks_for(most, 256), 148), (unsigned)count);
+    adam_many_kernel<<<grid, 256, 0, as_stream(stream)>>>(P);
+    return launch_status("adam_many_kernel");
+}
+
+int ffx_relu_bias_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pitch, const void* y, int32_t y_pitch,
+                           int32_t y_offset, float* dbias, void* stream) {
+    FFX_REQUIRE(voxels >= 1 && channels >= 8 && channels <= 128 && (channels & (channels - 1)) == 0 && dy && dbias &&
+                dy_pitch >= channels && dy_pitch % 8 == 0 && ((uintptr_t)dy & 15) == 0,
+                "ffx_relu_bias_backward: invalid arguments (channels: a power of two in [8, 128])");
+    FFX_REQUIRE(!y || (y_pitch >= y_offset + channels && y_offset >= 0 && y_pitch % 8 == 0 && y_offset % 8 == 0 &&
+                       ((uintptr_t)y & 15) == 0), "ffx_relu_bias_backward: invalid activation view");
+    const long long rows = 256 / (channels / 8);
+    const unsigned blocks = (unsigned)std::min<long long>((voxels + rows - 1) / rows, 148 * 4);
+    relu_bias_kernel<<<blocks, 256, 0, as_stream(stream)>>>(voxels, channels, (bf16*)dy, dy_pitch, (const bf16*)y,
+                                                            y_pitch, y_offset, dbias);
+    return launch_status("relu_bias_kernel");
 }
 
 int ffx_weight_transpose(int32_t taps, int32_t cin, int32_t cout, int32_t flip, const void* src, void* dst,
@@ -1466,8 +1712,22 @@ int ffx_mse_grad(int64_t voxels, const float* pred, int32_t pred_pitch, const fl
                  float inv_count, void* grad, double* loss, void* stream) {
     FFX_REQUIRE(voxels >= 1 && pred && target && grad && loss && pred_pitch >= 1 && ((uintptr_t)grad & 15) == 0,
                 "ffx_mse_grad: invalid arguments");
-    mse_kernel<<<blocks_for(voxels, 256), 256, 0, as_stream(stream)>>>(voxels, pred, pred_pitch, target, mask,
-                                                                        inv_count, (bf16*)grad, loss);
+    const unsigned blocks = (unsigned)std::min<long long>(blocks_for(voxels, 256), 148 * 8);
+    mse_kernel<<<blocks, 256, 0, as_stream(stream)>>>(voxels, pred, pred_pitch, target, mask, inv_count, nullptr,
+                                                      (bf16*)grad, loss);
+    return launch_status("mse_kernel");
+}
+
+int ffx_mse_grad_masked(int64_t voxels, const float* pred, int32_t pred_pitch, const float* target, const uint8_t* mask,
+                        int32_t* fluid, void* grad, double* loss, void* stream) {
+    FFX_REQUIRE(voxels >= 1 && voxels < (int64_t(1) << 31) && pred && target && mask && fluid && grad && loss &&
+                pred_pitch >= 1 && ((uintptr_t)grad & 15) == 0, "ffx_mse_grad_masked: invalid arguments");
+    const unsigned blocks = (unsigned)std::min<long long>(blocks_for(voxels, 256), 148 * 8);
+    fluid_count_kernel<<<blocks, 256, 0, as_stream(stream)>>>(voxels, mask, fluid);
+    int e = launch_status("fluid_count_kernel");
+    if (e) return e;
+    mse_kernel<<<blocks, 256, 0, as_stream(stream)>>>(voxels, pred, pred_pitch, target, mask, 0.f, fluid, (bf16*)grad,
+                                                      loss);
     return launch_status("mse_kernel");
 }
 

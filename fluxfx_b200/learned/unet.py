@@ -16,8 +16,8 @@ The decoder's concatenation buffers are written in place by both producers
 
 All work runs through ``libffx_core`` (``ffx_conv_forward_tma`` with
 ``ffx_conv_pack_weights``, ``ffx_conv_forward``, ``ffx_conv_weight_grad``,
-``ffx_relu_backward``, ``ffx_bias_grad``, ``ffx_weight_transpose``,
-``ffx_adam``, ``ffx_pack_input``, ``ffx_mse_grad``); torch only allocates.
+``ffx_relu_bias_backward``, ``ffx_weight_transpose``, ``ffx_adam_many``,
+``ffx_pack_input``, ``ffx_mse_grad_masked``); torch only allocates.
 The 3^3 layers (forward and data gradient) run on the TMA-staged tcgen05
 convolution by default; the stride-2, transposed and 1^3 layers on the
 mma.sync implicit GEMM.
@@ -56,8 +56,7 @@ class Layer:
         self.b = torch.zeros(cout, dtype=torch.float32, device=device)
         self.w16 = self.w.to(torch.bfloat16)
         self.wt16 = torch.empty((self.taps, cout, cin), dtype=torch.bfloat16, device=device)   # data-gradient weights
-        self.gw = torch.zeros_like(self.w)
-        self.gb = torch.zeros_like(self.b)
+        self.gw = self.gb = None      # gradients: views of the network's buffer
         self.mw, self.vw = torch.zeros_like(self.w), torch.zeros_like(self.w)
         self.mb, self.vb = torch.zeros_like(self.b), torch.zeros_like(self.b)
 
@@ -83,6 +82,12 @@ class UNet:
                 ('u0', 'up', c1, c0, True), ('c0a', 'conv3', 2 * c0, c0, True), ('c0b', 'conv3', c0, c0, True),
                 ('head', 'head', c0, HEAD_CHANNELS, False)]
         self.layers = [Layer(*s, device=device, gen=gen) for s in spec]
+        # every gradient in one buffer, cleared at once; the layers hold views of it
+        params = [t for l in self.layers for t in (l.w, l.b)]
+        self._gradients = torch.zeros(sum(t.numel() for t in params), dtype=torch.float32, device=device)
+        views = [v.view_as(t) for v, t in zip(self._gradients.split([t.numel() for t in params]), params)]
+        for l, gw, gb in zip(self.layers, views[0::2], views[1::2]):
+            l.gw, l.gb = gw, gb
         self.by_name = {l.name: l for l in self.layers}
         self.shape = None
         self.step_count = 0
@@ -134,6 +139,7 @@ class UNet:
         self.pred = torch.zeros((batch, D, H, W, HEAD_CHANNELS), dtype=torch.float32, device=dev)
         self.dpred = torch.zeros((batch, D, H, W, HEAD_CHANNELS), dtype=torch.bfloat16, device=dev)
         self.loss_acc = torch.zeros(1, dtype=torch.float64, device=dev)
+        self.fluid = torch.zeros(1, dtype=torch.int32, device=dev)
         self.shape = (batch, dims)
         self.batch = batch
         # (layer, level_in, input views, level_out, output tensor, out pitch, out offset)
@@ -252,15 +258,18 @@ class UNet:
         """MSE against `target` over fluid voxels, then gradients of every
         parameter (accumulated into layer.gw / layer.gb, zeroed here first)."""
         s = C.c_void_p(stream)
-        count = target.numel() if mask is None else int(target.numel() - int(mask.sum()))
         self.loss_acc.zero_()
-        self._call('ffx_mse_grad', target.numel(), _p(self.pred), HEAD_CHANNELS, _p(target), _p(mask),
-                   1.0 / max(count, 1), _p(self.dpred), _p(self.loss_acc), s)
-        for l in self.layers:
-            l.gw.zero_()
-            l.gb.zero_()
-        for g in self.grad.values():
-            g.zero_()
+        if mask is None:
+            self._call('ffx_mse_grad', target.numel(), _p(self.pred), HEAD_CHANNELS, _p(target), None,
+                       1.0 / max(target.numel(), 1), _p(self.dpred), _p(self.loss_acc), s)
+        else:
+            # the fluid voxels are counted on the device: nothing is read back
+            self.fluid.zero_()
+            self._call('ffx_mse_grad_masked', target.numel(), _p(self.pred), HEAD_CHANNELS, _p(target), _p(mask),
+                       _p(self.fluid), _p(self.dpred), _p(self.loss_acc), s)
+            self.calls += 1     # the count is a launch of its own
+        # (activation gradients need no clearing: each is written before it is added to or read)
+        self._gradients.zero_()
         for name, lin, ins, lout, out, pitch, offset in reversed(self.graph):
             layer = self.by_name[name]
             if name == 'head':
@@ -269,13 +278,12 @@ class UNet:
                 gfull = self.grad_of[id(out)]
                 gout = gfull.view(-1)[offset:]     # channel offset inside the (concatenated) buffer
                 gpitch = pitch
-                if layer.relu:
-                    self._call('ffx_relu_backward', self._voxels(lout), layer.cout, _p(gout), gpitch, _p(out), pitch,
-                               offset, s)
-            # weight and bias gradients
+            # the ReLU derivative and the bias gradient, then the weight gradient
+            relu = layer.relu and name != 'head'
+            self._call('ffx_relu_bias_backward', self._voxels(lout), layer.cout, _p(gout), gpitch,
+                       _p(out) if relu else None, pitch, offset, _p(layer.gb), s)
             c = self._conv(layer, lin, ins[0], lout, None, 0, 0)
             self._call('ffx_conv_weight_grad', C.byref(c), _p(gout), gpitch, _p(layer.gw), s)
-            self._call('ffx_bias_grad', self._voxels(lout), layer.cout, _p(gout), gpitch, _p(layer.gb), s)
             if name == 'e0a':
                 continue
             # data gradient into the input's gradient view
@@ -310,10 +318,11 @@ class UNet:
         self.step_count += 1
         self.weight_version += 1
         s = C.c_void_p(stream)
-        for l in self.layers:
-            for w, m, v, g, w16 in l.params():
-                self._call('ffx_adam', w.numel(), _p(w), _p(m), _p(v), _p(g), _p(w16), lr, beta1, beta2, eps,
-                           self.step_count, s)
+        params = [p for l in self.layers for p in l.params()]
+        slots = (N.FfxAdamSlot * len(params))(*[
+            (w.numel(), w.data_ptr(), m.data_ptr(), v.data_ptr(), g.data_ptr(),
+             w16.data_ptr() if w16 is not None else None) for w, m, v, g, w16 in params])
+        self._call('ffx_adam_many', len(slots), slots, lr, beta1, beta2, eps, self.step_count, s)
 
     # ------------------------------------------------------------- state
     def state_dict(self):

@@ -899,6 +899,10 @@ int ffx_relu_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pit
 /* dbias[c] += sum over voxels of g[v][c] (channels <= 128, dividing 256). */
 int ffx_bias_grad(int64_t voxels, int32_t channels, const void* g, int32_t pitch, float* dbias,
                   void* stream);
+/* Both in one pass: dy *= (y > 0) (y NULL: dy as it is), then dbias[c] += sum of dy.
+ * channels: a power of two in [8, 128]; pitches and offset multiples of 8, views on 16 bytes. */
+int ffx_relu_bias_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pitch, const void* y,
+                           int32_t y_pitch, int32_t y_offset, float* dbias, void* stream);
 /* Weights of the data-gradient convolution: dst[t][co][ci] = src[flip ? taps-1-t : t][ci][co]. */
 int ffx_weight_transpose(int32_t taps, int32_t cin, int32_t cout, int32_t flip, const void* src,
                          void* dst, void* stream);
@@ -906,6 +910,18 @@ int ffx_weight_transpose(int32_t taps, int32_t cin, int32_t cout, int32_t flip, 
  * receives the rounded weights. */
 int ffx_adam(int64_t n, float* w, float* m, float* v, const float* g, void* w_bf16, float lr,
              float beta1, float beta2, float eps, int32_t step, void* stream);
+/* ffx_adam of up to FFX_ADAM_SLOTS tensors in one launch (w_bf16 of a slot may be NULL). */
+#define FFX_ADAM_SLOTS 64
+typedef struct FfxAdamSlot {
+    int64_t n;
+    float* w;
+    float* m;
+    float* v;
+    const float* g;
+    void* w_bf16;
+} FfxAdamSlot;
+int ffx_adam_many(int32_t count, const FfxAdamSlot* slots, float lr, float beta1, float beta2, float eps,
+                  int32_t step, void* stream);
 /* Network input, 8 BF16 channels per voxel: scale * div, solid mask, zeros. */
 int ffx_pack_input(int64_t voxels, const float* div, const uint8_t* mask, float scale, void* out,
                    void* stream);
@@ -928,6 +944,10 @@ int ffx_unpack_channel_scaled(int64_t voxels, const float* src, int32_t pitch, c
  * channels per voxel) = its derivative in channel 0. */
 int ffx_mse_grad(int64_t voxels, const float* pred, int32_t pred_pitch, const float* target,
                  const uint8_t* mask, float inv_count, void* grad, double* loss, void* stream);
+/* The same with inv_count = 1 / max(fluid voxels, 1) counted on the device: *fluid
+ * (zeroed by the caller) is raised by voxels - the sum of the mask. */
+int ffx_mse_grad_masked(int64_t voxels, const float* pred, int32_t pred_pitch, const float* target,
+                        const uint8_t* mask, int32_t* fluid, void* grad, double* loss, void* stream);
 
 #ifdef __cplusplus
 }
