@@ -122,6 +122,13 @@ class FfxConv(C.Structure):
                 ('out_f32_pitch', i32)]
 
 
+WGRAD_LAYERS = 32
+
+
+class FfxWeightGrad(C.Structure):
+    _fields_ = [('conv', FfxConv), ('grad', vp), ('grad_pitch', i32), ('dweight', vp)]
+
+
 ADAM_SLOTS = 64
 
 
@@ -288,6 +295,7 @@ _PROTOTYPES = {
     'ffx_conv_pack_weights': (C.c_int, [P(FfxConv), vp, vp]),
     'ffx_conv_forward_tma': (C.c_int, [P(FfxConv), vp, vp]),
     'ffx_conv_weight_grad': (C.c_int, [P(FfxConv), vp, i32, vp, vp]),
+    'ffx_conv_weight_grad_many': (C.c_int, [i32, P(FfxWeightGrad), vp]),
     'ffx_relu_backward': (C.c_int, [i64, i32, vp, i32, vp, i32, i32, vp]),
     'ffx_bias_grad': (C.c_int, [i64, i32, vp, i32, vp, vp]),
     'ffx_weight_transpose': (C.c_int, [i32, i32, i32, i32, vp, vp, vp]),

@@ -890,14 +890,14 @@ __global__ void conv3_pack_kernel(const bf16* __restrict__ w, int cin, int cout,
 // voxels is 512 of them in a row, whatever the tile. So the tile is narrow (64
 // input by 16 or 32 output channels; a warp has 16 of the former and half of
 // the latter), a step is one or two MMAs long, and a layer of one chunk still
-// fills the SMs (64 -> 64 channels: 54 blocks). A stage is 64 voxels and up to
-// six are in flight, so a step never waits for its gathers, and a gather costs
+// fills the SMs (64 -> 64 channels: 54 blocks). A stage is 64 voxels and three
+// are in flight, so a step never waits for its gathers, and a gather costs
 // a dozen instructions: its tap is fixed per thread and its voxel's position
 // moves by carries, not divisions. Every accumulator sums its voxels in the
 // order of the 16-voxel steps, so a chunk's sums do not depend on the tile.
 // With a 128 x 64 tile, three 16-voxel stages and 64-bit divisions per gather a
 // step took 1.4 us and a layer 730 us.
-constexpr int kWgVox = 64, kWgK = 64, kWgStages = 6, kWgThreads = 256;
+constexpr int kWgVox = 64, kWgK = 64, kWgStages = 4, kWgThreads = 256;
 
 struct Wgrad {
     Conv a;
@@ -907,6 +907,8 @@ struct Wgrad {
     int chunk;
     int w, h, d;               // the GEMM row's grid (output voxels, or input voxels per parity class)
     int step_x, step_y, step_z;   // kWgVox rows further, in that grid
+    int nt, kind;              // output channels of a block (16 or 32), WgKind
+    int blocks_k, blocks_n, blocks_z;
 };
 
 // Position of a GEMM row that moves on by kWgVox rows at a time.
@@ -936,7 +938,7 @@ struct Walk {
 enum WgKind { kWgSame = 0, kWgStrided = 1, kWgTransposed = 2 };
 
 template <int NT, int KIND>
-__global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(const __grid_constant__ Wgrad P) {
+__device__ __forceinline__ void wgrad_block(const Wgrad& P, int block_k, int block_n, int block_z) {
     constexpr int AS = kWgK + 8, GS = NT + 8;      // bf16 per shared row (8 pad: conflict-free ldmatrix)
     constexpr int NW = NT / 2;                     // output channels of a warp
     constexpr int kRows = kWgThreads / 8;          // voxels that the block's gathers cover at once
@@ -945,9 +947,9 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(const __grid_con
     bf16* sG = sA + kWgStages * kWgVox * AS;
     const Conv& a = P.a;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int k0 = blockIdx.x * kWgK, n0 = blockIdx.y * NT;
-    const int cls = KIND == kWgTransposed ? (int)(blockIdx.z % 8) : 0;
-    const int split = KIND == kWgTransposed ? (int)(blockIdx.z / 8) : (int)blockIdx.z;
+    const int k0 = block_k * kWgK, n0 = block_n * NT;
+    const int cls = KIND == kWgTransposed ? block_z % 8 : 0;
+    const int split = KIND == kWgTransposed ? block_z / 8 : block_z;
     const int mb = split * P.chunk;
     const int rows = (int)min(a.rows - mb, (long long)P.chunk);
     const int stages = (rows + kWgVox - 1) / kWgVox;
@@ -1066,6 +1068,34 @@ __global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(const __grid_con
             atomicAdd(base + (size_t)k * a.cout + n, acc[nt][half * 2]);
             atomicAdd(base + (size_t)k * a.cout + n + 1, acc[nt][half * 2 + 1]);
         }
+    }
+}
+
+// The weight gradients of several layers in one launch: they depend on nothing
+// but finished activations and gradients, a layer's blocks all take one chain's
+// time, and most layers alone leave SMs idle.
+struct WgradMany {
+    int count;
+    int first[FFX_WGRAD_LAYERS + 1];     // first block of each layer
+    Wgrad layer[FFX_WGRAD_LAYERS];
+};
+
+__global__ void __launch_bounds__(kWgThreads) conv_wgrad_kernel(const __grid_constant__ WgradMany A) {
+    int k = 0;
+    while (k + 1 < A.count && (int)blockIdx.x >= A.first[k + 1]) ++k;
+    const Wgrad& P = A.layer[k];
+    int r = (int)blockIdx.x - A.first[k];
+    const int bk = r % P.blocks_k;
+    r /= P.blocks_k;
+    const int bn = r % P.blocks_n, bz = r / P.blocks_n;
+    if (P.nt == 16) {
+        if (P.kind == kWgSame) wgrad_block<16, kWgSame>(P, bk, bn, bz);
+        else if (P.kind == kWgStrided) wgrad_block<16, kWgStrided>(P, bk, bn, bz);
+        else wgrad_block<16, kWgTransposed>(P, bk, bn, bz);
+    } else {
+        if (P.kind == kWgSame) wgrad_block<32, kWgSame>(P, bk, bn, bz);
+        else if (P.kind == kWgStrided) wgrad_block<32, kWgStrided>(P, bk, bn, bz);
+        else wgrad_block<32, kWgTransposed>(P, bk, bn, bz);
     }
 }
 
@@ -1541,7 +1571,7 @@ int ffx_conv_timeouts(int32_t* out, int32_t reset) {
     return e;
 }
 
-int ffx_conv_weight_grad(const FfxConv* c, const void* grad, int32_t grad_pitch, float* dweight, void* stream) {
+static int make_wgrad(const FfxConv* c, const void* grad, int32_t grad_pitch, float* dweight, Wgrad& P) {
     Conv a;
     int e = make_conv(c, a);
     if (e) return e;
@@ -1551,7 +1581,7 @@ int ffx_conv_weight_grad(const FfxConv* c, const void* grad, int32_t grad_pitch,
     const long long splits = (a.rows + chunk - 1) / chunk;
     FFX_REQUIRE(splits * (a.transposed ? 8 : 1) < 65536 && a.rows < (1ll << 31),
                 "ffx_conv_weight_grad: too many voxels for one launch");
-    Wgrad P = {};
+    P = {};
     P.a = a;
     P.g = (const bf16*)grad;
     P.g_pitch = grad_pitch;
@@ -1563,32 +1593,45 @@ int ffx_conv_weight_grad(const FfxConv* c, const void* grad, int32_t grad_pitch,
     P.step_x = kWgVox % P.w;
     P.step_y = kWgVox / P.w % P.h;
     P.step_z = kWgVox / P.w / P.h;
-    // 16 output channels a block where the layer has no more, else 32
-    auto launch = [&](auto nt, auto kind) {
-        constexpr int NT = decltype(nt)::value, KIND = decltype(kind)::value;
-        constexpr int smem = kWgStages * kWgVox * (kWgK + 8 + NT + 8) * (int)sizeof(bf16);
-        static std::atomic<uint64_t> ready{0};
-        int dev = 0;
-        cudaError_t err = cudaGetDevice(&dev);
-        if (err == cudaSuccess && !(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
-            err = cudaFuncSetAttribute(conv_wgrad_kernel<NT, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (err == cudaSuccess) ready.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_release);
-        }
-        if (err != cudaSuccess) return cuda_status(err, "ffx_conv_weight_grad");
-        const dim3 grid((unsigned)((a.k_units * 8 + kWgK - 1) / kWgK), (unsigned)((a.cout + NT - 1) / NT),
-                        (unsigned)(splits * (a.transposed ? 8 : 1)));
-        conv_wgrad_kernel<NT, KIND><<<grid, kWgThreads, smem, as_stream(stream)>>>(P);
-        return launch_status("conv_wgrad_kernel");
-    };
-    const std::integral_constant<int, kWgSame> same;
-    const std::integral_constant<int, kWgStrided> strided;
-    const std::integral_constant<int, kWgTransposed> transposed;
-    const std::integral_constant<int, 16> narrow;
-    const std::integral_constant<int, 32> wide;
-    if (a.transposed) return a.cout <= 16 ? launch(narrow, transposed) : launch(wide, transposed);
-    if (a.stride == 1 && a.id == a.od && a.ih == a.oh && a.iw == a.ow)
-        return a.cout <= 16 ? launch(narrow, same) : launch(wide, same);
-    return a.cout <= 16 ? launch(narrow, strided) : launch(wide, strided);
+    P.nt = a.cout <= 16 ? 16 : 32;      // 16 output channels a block where the layer has no more
+    const bool same = a.stride == 1 && a.id == a.od && a.ih == a.oh && a.iw == a.ow;
+    P.kind = a.transposed ? kWgTransposed : (same ? kWgSame : kWgStrided);
+    P.blocks_k = (a.k_units * 8 + kWgK - 1) / kWgK;
+    P.blocks_n = (a.cout + P.nt - 1) / P.nt;
+    P.blocks_z = (int)(splits * (a.transposed ? 8 : 1));
+    return FFX_OK;
+}
+
+int ffx_conv_weight_grad_many(int32_t count, const FfxWeightGrad* layers, void* stream) {
+    FFX_REQUIRE(count >= 1 && count <= FFX_WGRAD_LAYERS && layers, "ffx_conv_weight_grad_many: invalid arguments");
+    WgradMany A;
+    A.count = count;
+    A.first[0] = 0;
+    long long blocks = 0;
+    for (int k = 0; k < count; ++k) {
+        Wgrad& P = A.layer[k];
+        if (int e = make_wgrad(&layers[k].conv, layers[k].grad, layers[k].grad_pitch, layers[k].dweight, P)) return e;
+        blocks += (long long)P.blocks_k * P.blocks_n * P.blocks_z;
+        FFX_REQUIRE(blocks < (1ll << 31), "ffx_conv_weight_grad_many: too many blocks for one launch");
+        A.first[k + 1] = (int)blocks;
+    }
+    constexpr int smem = kWgStages * kWgVox * (kWgK + 8 + 32 + 8) * (int)sizeof(bf16);
+    static std::atomic<uint64_t> ready{0};
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err == cudaSuccess && !(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
+        err = cudaFuncSetAttribute(conv_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err == cudaSuccess) ready.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_release);
+    }
+    if (err != cudaSuccess) return cuda_status(err, "ffx_conv_weight_grad_many");
+    conv_wgrad_kernel<<<(unsigned)blocks, kWgThreads, smem, as_stream(stream)>>>(A);
+    return launch_status("conv_wgrad_kernel");
+}
+
+int ffx_conv_weight_grad(const FfxConv* c, const void* grad, int32_t grad_pitch, float* dweight, void* stream) {
+    FFX_REQUIRE(c, "ffx_conv_weight_grad: invalid arguments");
+    const FfxWeightGrad one = {*c, grad, grad_pitch, dweight};
+    return ffx_conv_weight_grad_many(1, &one, stream);
 }
 
 int ffx_relu_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pitch, const void* y, int32_t y_pitch,

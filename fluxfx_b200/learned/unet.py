@@ -15,7 +15,7 @@ The decoder's concatenation buffers are written in place by both producers
 [C, 2C)), and their gradients likewise, so no copies are made.
 
 All work runs through ``libffx_core`` (``ffx_conv_forward_tma`` with
-``ffx_conv_pack_weights``, ``ffx_conv_forward``, ``ffx_conv_weight_grad``,
+``ffx_conv_pack_weights``, ``ffx_conv_forward``, ``ffx_conv_weight_grad_many``,
 ``ffx_relu_bias_backward``, ``ffx_weight_transpose``, ``ffx_adam_many``,
 ``ffx_pack_input``, ``ffx_mse_grad_masked``); torch only allocates.
 The 3^3 layers (forward and data gradient) run on the TMA-staged tcgen05
@@ -270,6 +270,7 @@ class UNet:
             self.calls += 1     # the count is a launch of its own
         # (activation gradients need no clearing: each is written before it is added to or read)
         self._gradients.zero_()
+        todo = []
         for name, lin, ins, lout, out, pitch, offset in reversed(self.graph):
             layer = self.by_name[name]
             if name == 'head':
@@ -278,12 +279,12 @@ class UNet:
                 gfull = self.grad_of[id(out)]
                 gout = gfull.view(-1)[offset:]     # channel offset inside the (concatenated) buffer
                 gpitch = pitch
-            # the ReLU derivative and the bias gradient, then the weight gradient
+            # the ReLU derivative and the bias gradient; the weight gradient waits for the others
             relu = layer.relu and name != 'head'
             self._call('ffx_relu_bias_backward', self._voxels(lout), layer.cout, _p(gout), gpitch,
                        _p(out) if relu else None, pitch, offset, _p(layer.gb), s)
-            c = self._conv(layer, lin, ins[0], lout, None, 0, 0)
-            self._call('ffx_conv_weight_grad', C.byref(c), _p(gout), gpitch, _p(layer.gw), s)
+            todo.append((self._conv(layer, lin, ins[0], lout, None, 0, 0), gout.data_ptr(), gpitch,
+                         layer.gw.data_ptr()))
             if name == 'e0a':
                 continue
             # data gradient into the input's gradient view
@@ -308,6 +309,7 @@ class UNet:
                 c = self._conv(layer, lout, g_view, lin, gin, ipitch, ioff, weight=layer.wt16, transposed=0,
                                ks=2, stride=2, pad=0, cout=layer.cin, bias=False, relu=False)
             self._run_conv((name, 'data'), c, s)
+        self._call('ffx_conv_weight_grad_many', len(todo), (N.FfxWeightGrad * len(todo))(*todo), s)
         return self.loss_acc
 
     def _voxels(self, level):

@@ -893,6 +893,15 @@ int ffx_conv_timeouts(int32_t* out, int32_t reset);
  * `grad` is the BF16 gradient of the convolution's output (ReLU already applied). */
 int ffx_conv_weight_grad(const FfxConv* conv, const void* grad, int32_t grad_pitch, float* dweight,
                          void* stream);
+/* The same for several layers in one launch. */
+#define FFX_WGRAD_LAYERS 32
+typedef struct FfxWeightGrad {
+    FfxConv conv;
+    const void* grad;
+    int32_t grad_pitch;
+    float* dweight;
+} FfxWeightGrad;
+int ffx_conv_weight_grad_many(int32_t count, const FfxWeightGrad* layers, void* stream);
 /* dy *= (y > 0) in place. */
 int ffx_relu_backward(int64_t voxels, int32_t channels, void* dy, int32_t dy_pitch, const void* y,
                       int32_t y_pitch, int32_t y_offset, void* stream);
