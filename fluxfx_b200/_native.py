@@ -62,6 +62,15 @@ class FfxGraphLevel(C.Structure):
                 ('coarse_scale', f32), ('links', vp)]
 
 
+GRAPH_PLAN_LEVELS = 10
+
+
+class FfxGraphPlan(C.Structure):
+    _fields_ = [('count', i32), ('pre0', i32), ('post0', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32),
+                ('omega', f32), ('inverse', vp), ('level', FfxGraphLevel * GRAPH_PLAN_LEVELS), ('blocks', i32),
+                ('tile', i32 * 2), ('tail', i32), ('shared_bytes', i32), ('workspace_bytes', i64), ('workspace', vp)]
+
+
 TAIL_LEVELS = 8
 MOVING_MAX = 8
 
@@ -288,6 +297,10 @@ _PROTOTYPES = {
     'ffx_graph_level0_edges': (C.c_int, [P(FfxGraphLevel), vp, vp]),
     'ffx_graph_links': (C.c_int, [P(FfxGraphLevel), vp, vp]),
     'ffx_graph_tail': (C.c_int, [P(FfxGraphTail), vp]),
+    'ffx_graph_plan': (C.c_int, [P(FfxGraphPlan)]),
+    'ffx_graph_plan_upload': (C.c_int, [P(FfxGraphPlan), vp]),
+    'ffx_graph_solve': (C.c_int, [P(FfxGraphPlan), vp, vp, i32, i32, C.c_double, i32, vp, vp]),
+    'ffx_graph_plan_timeouts': (C.c_int, [P(FfxGraphPlan), P(i32), vp]),
     'ffx_conv_forward': (C.c_int, [P(FfxConv), vp]),
     'ffx_conv_forward_tc': (C.c_int, [P(FfxConv), vp]),
     'ffx_conv_timeouts': (C.c_int, [P(i32), i32]),

@@ -4,7 +4,9 @@ Drop-in for FluxFX ``fluxfx/backend/solid_multigrid.py:7-93``. The Galerkin
 hierarchy of ``fluxfx/physics/solid_hierarchy.py:11-54`` is built on the device
 (``ffx_graph_coarsen`` per level, one flag readback per level at construction);
 level 0 stores one link byte per cell (``ffx_graph_links``) instead of
-conductances. The coarsest
+conductances. Solves of grids that fit the SMs' shared memory run in one
+launch, and so does the coarse part of the other grids' V-cycles
+(``ffx_graph_solve``). The coarsest
 level (<= 256 cells) is solved with an FP64 graph pseudoinverse. Residual +
 restriction and prolongation + first post-smoothing sweep are fused passes
 with results identical to the separate passes.
@@ -103,6 +105,9 @@ class SolidMultigridProjector(SolidPressureProjector):
         # (read back asynchronously) instead of waiting for them (coarse direct
         # solves are refreshed at once, as they need the new records on the host)
         self.defer_refresh_check = False
+        # solves that fit the chip's shared memory run in one launch, and the coarse
+        # part of the others' V-cycles does (ffx_graph_solve; same results)
+        self.use_resident = True
         # level-0 sweeps in fused pairs (ffx_graph_smooth2; same results; off: measured slower)
         self.fuse_sweeps = False
         # the device loop's convergence test also makes the next cycle's first
@@ -196,6 +201,53 @@ class SolidMultigridProjector(SolidPressureProjector):
             torch.cuda.synchronize(dev.device)
             self._free_loops()
         self._tail, self.tail_start = self._make_tail()
+        # resident plans by first level (0: whole solves), made when first asked for
+        self._residents = {}
+        self._coarse_first = None
+
+    def _resident(self, first):
+        """Plan of the levels from ``first`` on as one launch (ffx_graph_solve), or
+        None where they do not fit; its workspace is a tensor beside it."""
+        if first not in self._residents:
+            dev = self.device
+            plan = N.FfxGraphPlan()
+            levels = self.levels[first:]
+            entry = None
+            if 1 <= len(levels) <= N.GRAPH_PLAN_LEVELS and (first > 0 or len(levels) > 1):
+                plan.count = len(levels)
+                plan.pre, plan.post = self.coarse_pre, self.coarse_post
+                plan.pre0, plan.post0 = (self.pre_sweeps, self.post_sweeps) if first == 0 else (plan.pre, plan.post)
+                plan.last_sweeps, plan.omega = 80, 2.0 / 3.0
+                plan.inverse = self.coarse_matrix.data_ptr() if self.coarse_matrix is not None else None
+                for slot, level in enumerate(levels):
+                    plan.level[slot] = level['graph']
+                N.check(dev.lib.ffx_graph_plan(C.byref(plan)))
+                if plan.blocks:
+                    with dev.ordered():
+                        workspace = torch.zeros(plan.workspace_bytes, dtype=torch.uint8, device=dev.device)
+                    plan.workspace = workspace.data_ptr()
+                    N.check(dev.lib.ffx_graph_plan_upload(C.byref(plan), dev.s))
+                    entry = (plan, workspace)
+            self._residents[first] = entry
+        return self._residents[first]
+
+    def _coarse_resident(self):
+        """First level of the coarse part that runs as one launch, or None."""
+        if not self.use_resident:
+            return None
+        if self._coarse_first is None:
+            self._coarse_first = next((k for k in range(1, len(self.levels)) if self._resident(k)), -1)
+        return self._coarse_first if self._coarse_first > 0 else None
+
+    def _prepare_cycles(self):
+        """Makes the plan that a V-cycle's coarse part uses (it allocates, so before any capture)."""
+        self._coarse_resident()
+
+    def _cycle_sweeps(self):
+        """Sweeps of one V-cycle on all levels."""
+        last = len(self.levels) - 1
+        return (self.pre_sweeps + self.post_sweeps + (last - 1) * (self.coarse_pre + self.coarse_post) +
+                (0 if self.coarse_matrix is not None else 80))
 
     def _coarse_solve(self):
         """FP64 pseudoinverse of the coarsest level. A matrix of the same size is
@@ -289,7 +341,8 @@ class SolidMultigridProjector(SolidPressureProjector):
         coarse = sum(4 * 7 * prod(v['shape']) for v in self.levels[1:])
         direct = 8 * self.coarse_matrix.numel() if self.coarse_matrix is not None else 0
         links = self._links.numel() if self._links is not None else 0
-        return super().allocated_bytes + coarse + direct + links
+        resident = sum(e[1].numel() for e in self._residents.values() if e is not None)
+        return super().allocated_bytes + coarse + direct + links + resident
 
     def _fuse_cycle(self, level, zero_init, dot):
         """Whether this cycle runs its level-0 sweeps in fused pairs
@@ -365,13 +418,20 @@ class SolidMultigridProjector(SolidPressureProjector):
                 level['p'].zero_()
         self.smooth(level, pre, fuse)
         coarse = self.levels[index + 1]
-        tail = self.use_tail and index + 1 == self.tail_start
+        resident = index + 1 == self._coarse_resident()
+        tail = resident or (self.use_tail and index + 1 == self.tail_start)
         # the coarse iterate starts from zero: the restriction pass clears it
         # (the tail clears its own levels)
         dev.call('ffx_graph_residual_restrict_zero', C.byref(level['graph']), ptr(level['p']), ptr(level['rhs']),
                  ptr(coarse['rhs']), None if tail else ptr(coarse['p']), dev.s)
-        if tail:
+        if resident:
             # every level below runs inside one launch
+            plan = self._resident(index + 1)[0]
+            dev.call('ffx_graph_solve', C.byref(plan), ptr(coarse['p']), ptr(coarse['rhs']), 1, 1, 0.0, 0, None, dev.s)
+            below = len(self.levels) - index - 2
+            self.last_iterations += below * (self.coarse_pre + self.coarse_post) + (
+                0 if self.coarse_matrix is not None else 80)
+        elif tail:
             dev.call('ffx_graph_tail', C.byref(self._tail), dev.s)
             self.last_iterations += self._tail_sweeps()
         else:
@@ -518,6 +578,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         if len(self.levels) == 1:
             return super().solve_pressure(dt, previous_dt)
         warm = s.solid_warm_start and previous_dt is not None
+        from_zero = False
         if warm and s.learned_warm_start and s.learned_correction and self.learned is not None:
             # learned correction of the warm start: p += N(rhs - L p)
             self._learned_correction()
@@ -526,10 +587,15 @@ class SolidMultigridProjector(SolidPressureProjector):
                 raise ValueError('learned_warm_start needs a model: projector.attach_learned(LearnedWarmStart(...))')
             self.learned.guess(self.before, self.pressure)
         elif not (s.solid_warm_start and previous_dt is not None):
-            self.pressure.zero_()
+            from_zero = True
         self.levels[0]['p'], self.levels[0]['q'] = self.pressure, self.spare
         self.last_iterations = 0
         budget = s.pressure_cycles * (s.pressure_cold_multiplier if previous_dt is None else 1)
+        if self._solve_resident(budget, from_zero):
+            return
+        if from_zero:
+            self.pressure.zero_()
+        self._prepare_cycles()
         if s.pressure_method == 'PCG':
             scale = 0.0
             if s.pressure_tolerance > 0:
@@ -569,6 +635,39 @@ class SolidMultigridProjector(SolidPressureProjector):
                     self.last_cycles += 1
         self.pressure, self.spare = self.levels[0]['p'], self.levels[0]['q']
         self._host_total += self.last_cycles
+
+    def _solve_resident(self, budget, from_zero):
+        """Plain V-cycles, all of them in one launch; False where the solve does not
+        fit or another way of running it was asked for."""
+        s = self.settings
+        if (not self.use_resident or s.pressure_method != 'VCYCLE' or self.timer is not None or not self.use_graphs
+                or self.fuse_sweeps or not self._resident(0)):
+            return False
+        tolerance = s.pressure_tolerance > 0
+        if tolerance and not self.use_device_loop:
+            return False
+        self.device.call('ffx_graph_solve', C.byref(self._resident(0)[0]), ptr(self.pressure), ptr(self.before),
+                         0 if tolerance else budget, int(from_zero), float(s.pressure_tolerance),
+                         int(s.pressure_max_cycles), ptr(self._counters), self.device.s)
+        self._sweeps_per_cycle = self._cycle_sweeps()
+        if tolerance:
+            self._loops['resident'] = (None, *self._resident(0))      # this solve's loop on the device
+            self._cycles_on_device = True
+        else:
+            self.last_cycles = budget
+            self.last_iterations = budget * self._sweeps_per_cycle
+            self._host_total += budget
+        return True
+
+    def resident_timeouts(self):
+        """Waits of resident solves that gave up (0 unless the GPU was held up for seconds)."""
+        total = 0
+        for entry in self._residents.values():
+            if entry is not None:
+                count = N.i32(0)
+                N.check(self.device.lib.ffx_graph_plan_timeouts(C.byref(entry[0]), C.byref(count), self.device.s))
+                total += count.value
+        return total
 
     # ------------------------------------------------------ device-side loop
     def _device_solve(self, refine=False):
@@ -690,7 +789,8 @@ class SolidMultigridProjector(SolidPressureProjector):
 
     def _free_loops(self):
         for handle, _, _ in self._loops.values():
-            self.device.lib.ffx_loop_destroy(handle)
+            if handle is not None:      # a resident solve's loop is its plan
+                self.device.lib.ffx_loop_destroy(handle)
         self._loops = {}
 
     def gradient_links(self):
@@ -758,6 +858,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         self.learned = None
         self._links = None
         self._tail = None
+        self._residents = {}
         self.levels = []
         self.coarse_matrix = self.coarse_kernel = None
         super().close()

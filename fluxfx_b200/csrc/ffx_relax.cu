@@ -572,11 +572,6 @@ using resident::Params;
 constexpr int kHeaderWords = 128;      // exchange numbers of the blocks, the timeout counter
 constexpr int kSms = 148;
 
-int runs_of(int flat, int tz) {
-    const int groups = std::min(std::max(resident::kThreads / flat, 1), tz);
-    return (tz + groups - 1) / groups;
-}
-
 int64_t slots_of(const int32_t n[3]) { return (int64_t)(up4(n[0]) / 4) * n[1] * n[2]; }
 
 // float4 of shared memory of the levels from `first` on, whole, in one block.
@@ -610,7 +605,7 @@ int tile_fit(const FfxRelaxPlan& P, int dist, int ty, int tz) {
     const int x4 = up4(P.level[0].grid.n[0]) / 4;
     if (x4 * ty > resident::kThreads || x4 * (2 * (ty + tz) + 4) > resident::kThreads * resident::kRimItems) return -1;
     if (16 * tile_f4(P, dist, ty, tz, false) <= resident::kSmem) return 0;
-    if (16 * tile_f4(P, dist, ty, tz, true) <= resident::kSmem && runs_of(x4 * ty, tz) <= resident::kRun) return 1;
+    if (16 * tile_f4(P, dist, ty, tz, true) <= resident::kSmem) return 1;
     return -1;
 }
 

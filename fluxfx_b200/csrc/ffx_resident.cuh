@@ -22,7 +22,7 @@
 // relaxes 64 float4, of which the words' way through the L2 is about half.
 // Measured, us per sweep, a launch per sweep (T fused sweeps per launch) ->
 // resident: 75 x 61 x 93 5.5 (3.5) -> 2.0, 64^3 4.1 (3.4) -> 1.6, 127^3 12 (11)
-// -> 6.0; us per V(3,3) cycle: 128^3 250 (143) -> 90, 32^3 95 (40) -> 24.
+// -> 4.8; us per V(3,3) cycle: 128^3 250 (143) -> 73, 32^3 95 (40) -> 24.
 //
 // Blocks wait for one another, so the launch is cooperative (all blocks
 // resident at once); every wait is bounded: after kSpinLimit polls a block
@@ -36,7 +36,6 @@ namespace resident {
 constexpr int kThreads = 512;
 constexpr int kLevels = 12;
 constexpr int kTailSlots = 1024;
-constexpr int kRun = 8;              // planes of a thread's run where a level has one copy of its pressure
 constexpr int kRimItems = 4;         // float4 of the rim a thread takes in
 constexpr int kDirectCells = 512;
 constexpr int kSmem = 220 * 1024;
@@ -244,7 +243,7 @@ __device__ __forceinline__ void rim_items(const View& v, int (&from)[kRimItems],
 // sum; diag counts the open neighbours. A thread owns a run of float4 along z.
 // With two copies of the pressure a sweep goes from P to Q and the copies
 // change places (the caller flips the level by count's parity); with one copy
-// (ONE) a thread forms its run of at most kRun, meets the block, then writes it.
+// (ONE) it works in place.
 // With an exchange, the rim is current again after every sweep.
 template <bool MASK, bool ONE>
 __device__ __forceinline__ void relax(View& v, int level, const float2* kd, const unsigned* cls, bool zero, int count,
@@ -279,7 +278,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
     const int64_t copy = 4 * (int64_t)v.x4 * v.n[1] * v.n[2];
     const float wx = v.w[0], wy = v.w[1], wz = v.w[2];
     const bool left = x > 0, right = x + 1 < v.x4, rim_y = y == 0 || y == v.ty - 1;
-    auto formed = [&](const float4* P, int j, bool blank, float4& lo, float4& c) {
+    auto formed = [&](const float4* P, int j, bool blank, float4& lo, float4& c, float4 hi) {
         const int i = i0 + j * v.plane;
         const float4 r = v.R[r0 + j * v.flat];
         float4 k = k0, d = d0;
@@ -290,7 +289,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             if (gz == 0 || gz == v.n[2] - 1) weights_of(edge, kd, k, d);
         }
         if (blank) return make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w);
-        const float4 hi = P[i + v.plane], ym = P[i - v.x4], yp = P[i + v.x4];
+        const float4 ym = P[i - v.x4], yp = P[i + v.x4];
         const float* row = reinterpret_cast<const float*>(P) + 4 * i;
         const float xl = left ? row[-1] : 0.f, xr = right ? row[4] : 0.f;
         float4 o;
@@ -316,20 +315,22 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             c = v.P[i0];
         }
         if (ONE) {
-            float4 out[kRun];
-#pragma unroll
-            for (int j = 0; j < kRun; ++j)
-                if (j < mine) {
-                    out[j] = formed(v.P, j, blank, lo, c);
-                    publish(j, out[j]);
-                }
+            // a plane at a time: the values above the run are read before anything is
+            // written, and a plane is written when every thread has formed its part of it
+            const float4 top = mine > 0 && !blank ? v.P[i0 + mine * v.plane] : zero4();
             __syncthreads();
-#pragma unroll
-            for (int j = 0; j < kRun; ++j)
-                if (j < mine) v.P[i0 + j * v.plane] = out[j];
+            for (int j = 0; j < run; ++j) {
+                float4 o = zero4();
+                if (j < mine) {
+                    o = formed(v.P, j, blank, lo, c, j == mine - 1 ? top : v.P[i0 + (j + 1) * v.plane]);
+                    publish(j, o);
+                }
+                __syncthreads();
+                if (j < mine) v.P[i0 + j * v.plane] = o;
+            }
         } else {
             for (int j = 0; j < mine; ++j) {
-                const float4 o = formed(v.P, j, blank, lo, c);
+                const float4 o = formed(v.P, j, blank, lo, c, v.P[i0 + (j + 1) * v.plane]);
                 publish(j, o);
                 v.Q[i0 + j * v.plane] = o;
             }

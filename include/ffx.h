@@ -459,6 +459,42 @@ typedef struct FfxGraphTail {
 } FfxGraphTail;
 int ffx_graph_tail(const FfxGraphTail* tail, void* stream);
 
+/* ------------------------------------ resident collider multigrid */
+/* Whole V-cycle solves of a collider hierarchy (backend/solid_multigrid.py:46-76),
+ * or the coarse part of a V-cycle, in one cooperative launch with iterate and
+ * operator resident on the chip. Results are bit-identical to the separate passes.
+ * level[0] with links and edges == NULL: the mask's grid, whole solves. level[0]
+ * with edges: a coarse level; a "solve" is one V-cycle from zero of it and the
+ * levels below, for its right-hand side. */
+#define FFX_GRAPH_PLAN_LEVELS 10
+typedef struct FfxGraphPlan {
+    int32_t count;
+    int32_t pre0, post0;      /* sweeps on level[0] */
+    int32_t pre, post;        /* sweeps on the levels below */
+    int32_t last_sweeps;      /* sweeps of the coarsest level without a direct solve */
+    float omega;
+    const double* inverse;    /* dense FP64 inverse of the coarsest level (device), or NULL */
+    FfxGraphLevel level[FFX_GRAPH_PLAN_LEVELS];
+    /* filled by ffx_graph_plan */
+    int32_t blocks;           /* 0: the hierarchy does not fit */
+    int32_t tile[2], tail;
+    int32_t shared_bytes;     /* filled by ffx_graph_plan_upload */
+    int64_t workspace_bytes;
+    void* workspace;          /* caller's, 256-byte aligned, zeroed once; for one solve at a time */
+} FfxGraphPlan;
+/* Whether and how the hierarchy fits (host only; blocks = 0 when it does not). */
+int ffx_graph_plan(FfxGraphPlan* plan);
+/* Writes the plan's record into its workspace (waits for the stream). */
+int ffx_graph_plan_upload(FfxGraphPlan* plan, void* stream);
+/* cycles > 0: that many V-cycles. cycles == 0: V-cycles while fewer than max_cycles
+ * and max|rhs - L p| > tol * max|rhs| (decided in FP64 before each; a zero rhs gives
+ * a zero p), with counters (device) [cycles of this solve, += cycles, += decisions].
+ * from_zero: p is not read and starts from zero. */
+int ffx_graph_solve(const FfxGraphPlan* plan, float* p, const float* rhs, int32_t cycles, int32_t from_zero,
+                    double tol, int32_t max_cycles, int32_t* counters, void* stream);
+/* Bounded waits that gave up since the workspace was zeroed (waits for the stream). */
+int ffx_graph_plan_timeouts(const FfxGraphPlan* plan, int32_t* count, void* stream);
+
 /* Level-0 link bytes from the mask: bit 2a / 2a+1 = the face to the lower /
  * upper neighbour along axis a joins two fluid cells inside the domain, bit 6
  * = the cell is fluid. The level-0 conductances of
