@@ -347,6 +347,7 @@ _PROTOTYPES = {
     'ffx_batch_graph_free': (C.c_int, [vp]),
     'ffx_batch_stats': (C.c_int, [vp, P(FfxBatchStats), vp]),
     'ffx_batch_parity': (C.c_int, [vp]),
+    'ffx_batch_resident_first': (C.c_int, [vp]),
     'ffx_batch_destroy': (C.c_int, [vp]),
 }
 

@@ -5,8 +5,9 @@ No counterpart in the reference, whose solvers own one domain each
 ``DenseProjectedSmoke`` solvers (collider path, FP32, stand-alone V-cycles to
 a tolerance) and runs their steps through ``libffx_core``'s batched plan
 (``ffx_batch_*``): one persistent launch per pass over every domain, the
-pressure solve as a conditional WHILE node of a CUDA graph that stops when
-every domain has converged, and each domain's next time step
+pressure solves in one launch where all domains fit the SMs' shared memory,
+else as a conditional WHILE node of a CUDA graph that stops when every domain
+has converged, and each domain's next time step
 ``min(dt_max, cfl * cell / max|u|)`` computed on the device, so a run of many
 steps is one graph launch with no host round trip. Each domain's fields after
 a batched run are bit-identical to stepping that solver alone (from a reset)
@@ -204,10 +205,14 @@ class BatchedSmoke:
         pre, post = doms[0].pre, doms[0].post
         coarse = int(any(d.tail_start >= 0 for d in doms)) + int(any(d.tail_start < 0 and d.inverse for d in doms))
         coarse += 80 * int(any(d.tail_start < 0 and not d.inverse for d in doms))
+        first = self.lib.ffx_batch_resident_first(self.plan)
+        if first == 1:      # level 0 by passes, the levels below in one launch
+            k, coarse = 1, 1
         cycle = k * (pre + 1) + coarse + k * post
         vc = int(any(d.velocity_corrected for d in doms))
         sc = int(any(d.scalar_corrected for d in doms))
-        return (vc + 3) + (1 + 2 * sc + 1) + 1 + iterations * (2 + cycle)
+        solve = 2 if first == 0 else iterations * (2 + cycle)
+        return (vc + 3) + (1 + 2 * sc + 1) + 1 + solve
 
     # ------------------------------------------------------------ autotuning
     def signature(self):

@@ -785,6 +785,8 @@ __global__ void __launch_bounds__(kThreads, 1) graph_resident_kernel(const Domai
     for (int i = tid; i < (int)(sizeof(Domain) / 4); i += kThreads)
         reinterpret_cast<int*>(&D)[i] = __ldg(reinterpret_cast<const int*>(domains + which) + i);
     __syncthreads();
+    // coarse parts: a domain that has converged takes no part in the cycle
+    if (!LINKS && A.batched && D.state->done) return;
     const int block = (int)blockIdx.x - D.first_block;
     const bool tail = block == D.gy * D.gz;
     const int clear = tail ? D.tail_f4 : D.tile_f4;

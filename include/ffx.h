@@ -882,6 +882,10 @@ int ffx_batch_graph_free(void* graph_exec);
 int ffx_batch_stats(const FfxBatchPlan* plan, FfxBatchStats* out, void* stream);
 /* Current parity: 0 = density[0]/temperature[0] hold the fields. */
 int ffx_batch_parity(const FfxBatchPlan* plan);
+/* First multigrid level that the plan's solves run in one launch over all
+ * domains: 0 (whole solves), 1 (the coarse part of each cycle), or -1 (neither
+ * fits the chip's shared memory: a launch per pass). */
+int ffx_batch_resident_first(const FfxBatchPlan* plan);
 int ffx_batch_destroy(FfxBatchPlan* plan);
 
 /* ------------------------------------------------- learned warm start (a18) */
