@@ -20,14 +20,19 @@ constexpr int kThreads = 256;
 // kernels: the register budget against the warps resident to hide the
 // gathers' latency, chosen by measurement at 256^3 (a build can override
 // each with -DFFX_MINB_<KERNEL>=n; 0 leaves the choice to the compiler).
+// us at 256^3 BF16 with colliders by the number of blocks: velocity 4: 1670,
+// 5: 1558, 6: 1474, 7: 1442 (but 211 for 204 at 96 x 80 x 112); predictor 4: 1241,
+// 6: 1142, 8: 1145; reverse 4: 556, 5: 500, 6: 474; final scalars 3: 819, 4: 651,
+// 6: 631 (but 42 for 37); forward scalars 5: 416, 6: 397, left to the compiler
+// 389 (but 30 for 27 at 128 x 96 x 112 without colliders).
 #ifndef FFX_MINB_PREDICTOR
 #define FFX_MINB_PREDICTOR 8
 #endif
 #ifndef FFX_MINB_VELOCITY
-#define FFX_MINB_VELOCITY 5
+#define FFX_MINB_VELOCITY 6
 #endif
 #ifndef FFX_MINB_SCALAR_PREDICTOR
-#define FFX_MINB_SCALAR_PREDICTOR 0
+#define FFX_MINB_SCALAR_PREDICTOR 6
 #endif
 #ifndef FFX_MINB_SCALARS
 #define FFX_MINB_SCALARS 4
@@ -69,64 +74,23 @@ __device__ __forceinline__ bool face_coords(const Blk& b, const Dev& d, FaceIdx&
     f.sz = d.nz + (f.axis == 2);
     f.x = b.x * b.bw + b.ox;
     f.y = b.y * b.bh + b.oy;
+    if (f.sx - b.x * b.bw == 1) {
+        // a tile of one column (the face beyond a row of whole tiles): every bw-th
+        // such tile takes bw tiles' rows, instead of one lane in each warp of all
+        f.x = b.x * b.bw;
+        f.y = b.y % b.bw ? f.sy : b.y * b.bh + b.oy * b.bw + b.ox;
+    }
     if (f.x >= f.sx || f.y >= f.sy || f.z >= f.sz) return false;
     f.i = f.x + f.sx * (f.y + f.sy * f.z);
     return true;
 }
 
-// Midpoint backtrace p -> departure (transport_face.glsl:8-17 and the same
-// lines of every advection shader); clipped at colliders when MASK.
-template <typename T, bool MASK, bool P2 = false>
-__device__ __forceinline__ F3 backtrace(const Dev& d, const Faces<T>& F, const uint8_t* solid, const uint8_t* halo,
-                                        F3 p, F3 v0,
-                                        float dt) {
-    float s = 0.5f * dt;
-    F3 mid = {p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z};
-    if (MASK) mid = clip_solid_trace<P2>(d, solid, halo, p, mid);
-    F3 vm = velocity_at<T, P2>(d, F, mid);
-    F3 dep = {p.x - dt * vm.x, p.y - dt * vm.y, p.z - dt * vm.z};
-    if (MASK) dep = clip_solid_trace<P2>(d, solid, halo, p, dep);
-    return dep;
-}
-
-// Closed scalar sample (closed_sample.glsl:7-29).
-template <typename T, bool MASK>
-__device__ __forceinline__ float sample_closed(const Dev& d, const uint8_t* solid, const T* __restrict__ f,
-                                               float qx, float qy, float qz) {
-    float bx = floorf(qx), by = floorf(qy), bz = floorf(qz);
-    float fx = qx - bx, fy = qy - by, fz = qz - bz;
-    int ix = floor_int(qx), iy = floor_int(qy), iz = floor_int(qz);
-    int x0 = min(max(ix, 0), d.nx - 1), x1 = min(max(ix + 1, 0), d.nx - 1);
-    int y0 = min(max(iy, 0), d.ny - 1), y1 = min(max(iy + 1, 0), d.ny - 1);
-    int z0 = min(max(iz, 0), d.nz - 1), z1 = min(max(iz + 1, 0), d.nz - 1);
-    if (MASK) {
-        int xs[2] = {x0, x1}, ys[2] = {y0, y1}, zs[2] = {z0, z1};
-        float value = 0.f, total = 0.f;
-        for (int oz = 0; oz < 2; ++oz) {
-            float wz = oz ? fz : 1.f - fz;
-            for (int oy = 0; oy < 2; ++oy) {
-                float wy = oy ? fy : 1.f - fy;
-                for (int ox = 0; ox < 2; ++ox) {
-                    float wx = ox ? fx : 1.f - fx;
-                    int c = cidx(d, xs[ox], ys[oy], zs[oz]);
-                    if (__ldg(solid + c)) continue;
-                    float weight = wx * wy * wz;
-                    value = value + weight * Store<T>::ld(f, c);
-                    total = total + weight;
-                }
-            }
-        }
-        return total > 1e-8f ? value / total : 0.f;
-    }
-    float f000 = Store<T>::ld(f, cidx(d, x0, y0, z0)), f100 = Store<T>::ld(f, cidx(d, x1, y0, z0));
-    float f010 = Store<T>::ld(f, cidx(d, x0, y1, z0)), f110 = Store<T>::ld(f, cidx(d, x1, y1, z0));
-    float f001 = Store<T>::ld(f, cidx(d, x0, y0, z1)), f101 = Store<T>::ld(f, cidx(d, x1, y0, z1));
-    float f011 = Store<T>::ld(f, cidx(d, x0, y1, z1)), f111 = Store<T>::ld(f, cidx(d, x1, y1, z1));
-    float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    float a0 = f000 * gx + f100 * fx, a1 = f010 * gx + f110 * fx;
-    float b0 = f001 * gx + f101 * fx, b1 = f011 * gx + f111 * fx;
-    float zz0 = a0 * gy + a1 * fy, zz1 = b0 * gy + b1 * fy;
-    return zz0 * gz + zz1 * fz;
+// Midpoint backtrace p -> departure (transport_face.glsl:8-17) without colliders.
+template <typename T>
+__device__ __forceinline__ F3 backtrace(const Dev& d, const Faces<T>& F, F3 p, F3 v0, float dt) {
+    const float s = 0.5f * dt;
+    const F3 vm = velocity_at(d, F, F3{p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z});
+    return F3{p.x - dt * vm.x, p.y - dt * vm.y, p.z - dt * vm.z};
 }
 
 // The time step of a pass: the launch parameter, or the value a device-side
@@ -174,8 +138,18 @@ __device__ __forceinline__ GlobalSampler<FaceFields<T>> face_sampler(const Dev& 
     return GlobalSampler<FaceFields<T>>{FaceFields<T>{d, F, second}};
 }
 
-template <typename T, bool MASK, bool P2, class Smp>
-__device__ __forceinline__ void face_predictor_face(const PredParams<T>& P, const FaceIdx& f, const Smp& smp) {
+// The body once per axis: the field pointers, sizes and offsets it depends on
+// are then known when compiling (blocks hold faces of one axis).
+template <class Body>
+__device__ __forceinline__ void by_axis(int axis, Body&& body) {
+    if (axis == 0) body(std::integral_constant<int, 0>());
+    else if (axis == 1) body(std::integral_constant<int, 1>());
+    else body(std::integral_constant<int, 2>());
+}
+
+template <int AXIS, typename T, bool MASK, bool P2, class Smp>
+__device__ __forceinline__ void face_predictor_axis(const PredParams<T>& P, FaceIdx f, const Smp& smp) {
+    f.axis = AXIS;
     const Dev& d = P.d;
     const uint8_t* __restrict__ solid = P.solid;
     const uint8_t* __restrict__ halo = P.halo;
@@ -191,10 +165,10 @@ __device__ __forceinline__ void face_predictor_face(const PredParams<T>& P, cons
     }
     float ox = f.axis == 0 ? 0.f : 0.5f, oy = f.axis == 1 ? 0.f : 0.5f, oz = f.axis == 2 ? 0.f : 0.5f;
     F3 p = {((float)f.x + ox) * d.h[0], ((float)f.y + oy) * d.h[1], ((float)f.z + oz) * d.h[2]};
-    F3 v0 = start_velocity_face<P2>(d, smp, p, f.axis, f.x, f.y, f.z);
+    F3 v0 = start_velocity_face<MASK, P2>(d, smp, p, f.axis, f.x, f.y, f.z);
     F3 dep = backtrace_s<MASK, P2>(d, smp, solid, halo, p, v0, dt, cv);
-    float value = smp.sample(f.axis, dv_h<P2>(d, dep.x, 0) - ox, dv_h<P2>(d, dep.y, 1) - oy,
-                             dv_h<P2>(d, dep.z, 2) - oz);
+    float value = smp.template sample<MASK>(f.axis, cells<MASK, P2>(d, dep.x, 0) - ox, cells<MASK, P2>(d, dep.y, 1) - oy,
+                             cells<MASK, P2>(d, dep.z, 2) - oz);
     Store<T>::st(out, f.i, value);
     if (float* D = P.dep[f.axis]) {
         const int nf = P.nf[f.axis];
@@ -210,6 +184,11 @@ __device__ __forceinline__ void face_predictor_face(const PredParams<T>& P, cons
         D[f.i + (kV0 + 1) * nf] = v0.y;
         D[f.i + (kV0 + 2) * nf] = v0.z;
     }
+}
+
+template <typename T, bool MASK, bool P2, class Smp>
+__device__ __forceinline__ void face_predictor_face(const PredParams<T>& P, const FaceIdx& f, const Smp& smp) {
+    by_axis(f.axis, [&](auto a) { face_predictor_axis<decltype(a)::value, T, MASK, P2>(P, f, smp); });
 }
 
 template <typename T, bool MASK, bool P2>
@@ -246,10 +225,10 @@ struct VelParams {
     SrcDev src;
 };
 
-template <typename T, bool MASK, bool P2, class Smp>
-__device__ __forceinline__ void advect_velocity_face(const VelParams<T>& P, const FaceIdx& f, const Smp& smp) {
+template <int axis, typename T, bool MASK, bool P2, class Smp>
+__device__ __forceinline__ void advect_velocity_axis(const VelParams<T>& P, FaceIdx f, const Smp& smp) {
     const Dev& d = P.d;
-    const int axis = f.axis;
+    f.axis = axis;
     if (P.apply_walls) {
         // a boundary face ends as its wall value whatever was advected into it
         // (the wall condition below), so its advection is skipped
@@ -283,16 +262,16 @@ __device__ __forceinline__ void advect_velocity_face(const VelParams<T>& P, cons
             dep = {__ldg(D + f.i), __ldg(D + f.i + nf), __ldg(D + f.i + 2 * nf)};
             v0 = {__ldg(D + f.i + kV0 * nf), __ldg(D + f.i + (kV0 + 1) * nf), __ldg(D + f.i + (kV0 + 2) * nf)};
         } else {
-            v0 = start_velocity_face<P2>(d, smp, p, axis, f.x, f.y, f.z);
+            v0 = start_velocity_face<MASK, P2>(d, smp, p, axis, f.x, f.y, f.z);
             dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
         }
         const T* orig = axis == 0 ? P.F.u : (axis == 1 ? P.F.v : P.F.w);
         const T* pred = axis == 0 ? P.P.u : (axis == 1 ? P.P.v : P.P.w);
-        float qx = dv_h<P2>(d, dep.x, 0) - off[0], qy = dv_h<P2>(d, dep.y, 1) - off[1],
-              qz = dv_h<P2>(d, dep.z, 2) - off[2];
+        float qx = cells<MASK, P2>(d, dep.x, 0) - off[0], qy = cells<MASK, P2>(d, dep.y, 1) - off[1],
+              qz = cells<MASK, P2>(d, dep.z, 2) - off[2];
         // the predictor's sample at the same departure point: the stored value
         // (FP32) or its unrounded copy in the fourth trace plane (BF16)
-        float low = !reuse ? smp.sample(axis, qx, qy, qz)
+        float low = !reuse ? smp.template sample<MASK>(axis, qx, qy, qz)
                            : (sizeof(T) == 4 ? Store<T>::ld(pred, f.i) : __ldg(P.dep[axis] + f.i + 3 * P.nf[axis]));
         value = low;
         if (P.corrected) {
@@ -305,15 +284,15 @@ __device__ __forceinline__ void advect_velocity_face(const VelParams<T>& P, cons
             }
             float s = 0.5f * dt;
             F3 mid2 = {p.x + s * v0.x, p.y + s * v0.y, p.z + s * v0.z};
-            F3 vm2 = velocity_s<P2>(d, smp, mid2);
+            F3 vm2 = velocity_s<MASK, P2>(d, smp, mid2);
             F3 arr = {p.x + dt * vm2.x, p.y + dt * vm2.y, p.z + dt * vm2.z};
             bool ok = !(dep.x < lob[0] || dep.y < lob[1] || dep.z < lob[2] || dep.x > hib[0] || dep.y > hib[1] ||
                         dep.z > hib[2] || arr.x < lob[0] || arr.y < lob[1] || arr.z < lob[2] || arr.x > hib[0] ||
                         arr.y > hib[1] || arr.z > hib[2]);
             if (MASK && ok) ok = safe_correction_from<P2>(d, P.solid, P.halo, cv, p, dep, mid2, arr);
             if (ok) {
-                float pa = smp.sample(3 + axis, dv_h<P2>(d, arr.x, 0) - off[0], dv_h<P2>(d, arr.y, 1) - off[1],
-                                      dv_h<P2>(d, arr.z, 2) - off[2]);
+                float pa = smp.template sample<MASK>(3 + axis, cells<MASK, P2>(d, arr.x, 0) - off[0], cells<MASK, P2>(d, arr.y, 1) - off[1],
+                                      cells<MASK, P2>(d, arr.z, 2) - off[2]);
                 float val = Store<T>::ld(pred, f.i) + 0.5f * (Store<T>::ld(orig, f.i) - pa);
                 // min / max of the 8 corners around the departure point, clamped to the grid
                 float lo, hi;
@@ -362,6 +341,11 @@ __device__ __forceinline__ void advect_velocity_face(const VelParams<T>& P, cons
         if (c == 0 || c == n - 1 || blocked) value = wall_value(P.walls, axis, f.i);
     }
     Store<T>::st(P.out[axis], f.i, value);
+}
+
+template <typename T, bool MASK, bool P2, class Smp>
+__device__ __forceinline__ void advect_velocity_face(const VelParams<T>& P, const FaceIdx& f, const Smp& smp) {
+    by_axis(f.axis, [&](auto a) { advect_velocity_axis<decltype(a)::value, T, MASK, P2>(P, f, smp); });
 }
 
 template <typename T, bool MASK, bool P2>
@@ -491,10 +475,10 @@ dim3 tiled_grid(int nx, int ny, int nz, int zchunk) {
 
 // Whether the transport passes run tiled (ffx_set_transport_tiling). Off by
 // default: on the 256^3 collider scene the tiled forms measured slower than the
-// gathers (face predictor 1.98 vs 1.68 ms, velocity 2.98 vs 2.44, scalar
-// predictor + reverse 2.21 vs 1.30, scalar final 1.51 vs 1.01): the passes are
-// bound by instruction issue, and staging adds instructions and a block
-// barrier per slice without removing arithmetic.
+// gathers, both with clamped corners one by one (face predictor 1.98 vs 1.68 ms,
+// velocity 2.98 vs 2.44, scalar predictor + reverse 2.21 vs 1.30, scalar final
+// 1.51 vs 1.01): the passes are bound by instruction issue, and staging adds
+// instructions and a block barrier per slice without removing arithmetic.
 int g_tiling = 0;
 
 // P0.3 plain face self-advection (mac_advect_velocity.glsl).
@@ -507,7 +491,7 @@ __global__ void __launch_bounds__(kThreads) mac_advect_velocity_kernel(Dev d, Fa
     F3 p = {((float)f.x + ox) * d.e[0] / d.nf[0], ((float)f.y + oy) * d.e[1] / d.nf[1],
             ((float)f.z + oz) * d.e[2] / d.nf[2]};
     F3 v0 = velocity_at(d, F, p);
-    F3 dep = backtrace<T, false>(d, F, nullptr, nullptr, p, v0, dt);
+    F3 dep = backtrace(d, F, p, v0, dt);
     F3 v = velocity_at(d, F, dep);
     T* out = f.axis == 0 ? ou : (f.axis == 1 ? ov : ow);
     Store<T>::st(out, f.i, comp(v, f.axis));
@@ -590,7 +574,7 @@ __device__ __forceinline__ void scalar_transport_cell(const ScalarXport<T>& P, i
         return;
     }
     F3 p = {((float)x + 0.5f) * d.h[0], ((float)y + 0.5f) * d.h[1], ((float)z + 0.5f) * d.h[2]};
-    F3 v0 = start_velocity_s<P2>(d, smp, p, 2 * x + 1, 2 * y + 1, 2 * z + 1);
+    F3 v0 = start_velocity_cell<MASK, P2>(d, smp, p, x, y, z);
     F3 dep;
     if (DECIDE) {
         // backtrace_s, keeping the unclipped midpoint and departure point: with
@@ -601,11 +585,11 @@ __device__ __forceinline__ void scalar_transport_cell(const ScalarXport<T>& P, i
         const float dtr = step_dt(P), s = 0.5f * dtr;
         const F3 mid = {p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z};
         const F3 midc = MASK ? clip_from<P2>(d, P.solid, P.halo, cv, p, mid) : mid;
-        const F3 vm = velocity_s<P2>(d, smp, midc);
+        const F3 vm = velocity_s<MASK, P2>(d, smp, midc);
         F3 arr = {p.x - dtr * vm.x, p.y - dtr * vm.y, p.z - dtr * vm.z};
         dep = MASK ? clip_from<P2>(d, P.solid, P.halo, cv, p, arr) : arr;
         if (!same_bits(midc, mid)) {
-            const F3 vm2 = velocity_s<P2>(d, smp, mid);
+            const F3 vm2 = velocity_s<MASK, P2>(d, smp, mid);
             arr = {p.x - dtr * vm2.x, p.y - dtr * vm2.y, p.z - dtr * vm2.z};
         }
         const F3 fdep = {__ldg(P.fdep + i), __ldg(P.fdep + i + P.n), __ldg(P.fdep + i + 2 * P.n)};
@@ -613,8 +597,8 @@ __device__ __forceinline__ void scalar_transport_cell(const ScalarXport<T>& P, i
     } else {
         dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, step_dt(P), cv);
     }
-    float qx = dv_h<P2>(d, dep.x, 0) - 0.5f, qy = dv_h<P2>(d, dep.y, 1) - 0.5f,
-          qz = dv_h<P2>(d, dep.z, 2) - 0.5f;
+    float qx = cells<MASK, P2>(d, dep.x, 0) - 0.5f, qy = cells<MASK, P2>(d, dep.y, 1) - 0.5f,
+          qz = cells<MASK, P2>(d, dep.z, 2) - 0.5f;
     const auto S = smp.template closed<MASK>(P.solid, qx, qy, qz, clear && near_start(d, p, dep));
     for (int c = 0; c < P.count; ++c) Store<T>::st(P.out[c], i, smp.template apply<MASK>(3 + c, S));
     if (P.dep) {
@@ -638,7 +622,7 @@ __global__ void FFX_LB_SCALAR_PREDICTOR scalar_transport_kernel(const __grid_con
 }
 
 #ifndef FFX_MINB_SCALAR_REVERSE
-#define FFX_MINB_SCALAR_REVERSE 5
+#define FFX_MINB_SCALAR_REVERSE 6
 #endif
 #if FFX_MINB_SCALAR_REVERSE > 0
 #define FFX_LB_SCALAR_REVERSE __launch_bounds__(kThreads, FFX_MINB_SCALAR_REVERSE)
@@ -701,12 +685,12 @@ __device__ __forceinline__ void advect_scalars_cell(const ScalarFinal<T>& P, int
     // the reverse pass decided the correction (scalar_transport_cell with ok)
     const bool decided = reuse && P.ok != nullptr;
     F3 v0 = {0.f, 0.f, 0.f};
-    if (!decided) v0 = start_velocity_s<P2>(d, smp, p, 2 * x + 1, 2 * y + 1, 2 * z + 1);
+    if (!decided) v0 = start_velocity_cell<MASK, P2>(d, smp, p, x, y, z);
     F3 dep;
     if (reuse) dep = {__ldg(P.dep + i), __ldg(P.dep + i + P.n), __ldg(P.dep + i + 2 * P.n)};
     else dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
-    float qx = dv_h<P2>(d, dep.x, 0) - 0.5f, qy = dv_h<P2>(d, dep.y, 1) - 0.5f,
-          qz = dv_h<P2>(d, dep.z, 2) - 0.5f;
+    float qx = cells<MASK, P2>(d, dep.x, 0) - 0.5f, qy = cells<MASK, P2>(d, dep.y, 1) - 0.5f,
+          qz = cells<MASK, P2>(d, dep.z, 2) - 0.5f;
     bool ok = false;
     if (decided) {
         ok = __ldg(P.ok + i) != 0;
@@ -714,7 +698,7 @@ __device__ __forceinline__ void advect_scalars_cell(const ScalarFinal<T>& P, int
         // correct_scalar.glsl:1-21
         float s = 0.5f * dt;
         F3 mid2 = {p.x + s * v0.x, p.y + s * v0.y, p.z + s * v0.z};
-        F3 vm2 = velocity_s<P2>(d, smp, mid2);
+        F3 vm2 = velocity_s<MASK, P2>(d, smp, mid2);
         F3 arr = {p.x + dt * vm2.x, p.y + dt * vm2.y, p.z + dt * vm2.z};
         ok = scalar_correction_ok<MASK, P2>(d, P.solid, P.halo, cv, p, dep, mid2, arr);
     }
@@ -888,7 +872,7 @@ __global__ void mac_advect_density_kernel(OpenParams P, Faces<T> F, const T* in,
     const int i = cidx(d, x, y, z);
     F3 p = {((float)x + 0.5f) * d.h[0], ((float)y + 0.5f) * d.h[1], ((float)z + 0.5f) * d.h[2]};
     F3 v0 = velocity_at(d, F, p);
-    F3 dep = backtrace<T, false>(d, F, nullptr, nullptr, p, v0, P.dt);
+    F3 dep = backtrace(d, F, p, v0, P.dt);
     float value = sample_zero(d, in, dep.x / d.h[0] - 0.5f, dep.y / d.h[1] - 0.5f, dep.z / d.h[2] - 0.5f) *
                   expf(-P.decay * P.dt);
     F3 off = {p.x - P.center.x, p.y - P.center.y, p.z - P.center.z};

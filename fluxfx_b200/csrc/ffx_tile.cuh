@@ -78,7 +78,7 @@ __device__ __forceinline__ Corners corners(const Window& w, int k, int ix, int i
 }
 
 // sample_face (mac_sample.glsl:2-19) of field k from the window, else `g`.
-template <typename T>
+template <bool EXACT, typename T>
 __device__ __forceinline__ float sample(const Window& w, int k, const T* __restrict__ g, int sx, int sy, int sz,
                                         float qx, float qy, float qz) {
     qx = fminf(fmaxf(qx, 0.f), (float)(sx - 1));
@@ -86,50 +86,25 @@ __device__ __forceinline__ float sample(const Window& w, int k, const T* __restr
     qz = fminf(fmaxf(qz, 0.f), (float)(sz - 1));
     const float bx = floorf(qx), by = floorf(qy), bz = floorf(qz);
     const int ix = (int)bx, iy = (int)by, iz = (int)bz;
-    if (!inside(w, ix, iy, iz)) return sample_face(g, sx, sy, sz, qx, qy, qz);
-    const float fx = qx - bx, fy = qy - by, fz = qz - bz;
+    if (!inside(w, ix, iy, iz)) return sample_face<EXACT>(g, sx, sy, sz, qx, qy, qz);
     const Corners c = corners(w, k, ix, iy, iz);
-    const float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    float v = 0.f;
-    v = v + gx * gy * gz * c.c0[0];
-    v = v + fx * gy * gz * c.c0[1];
-    v = v + gx * fy * gz * c.c0[kPitch];
-    v = v + fx * fy * gz * c.c0[kPitch + 1];
-    v = v + gx * gy * fz * c.c1[0];
-    v = v + fx * gy * fz * c.c1[1];
-    v = v + gx * fy * fz * c.c1[kPitch];
-    v = v + fx * fy * fz * c.c1[kPitch + 1];
-    return v;
+    const float v[8] = {c.c0[0], c.c0[1], c.c0[kPitch], c.c0[kPitch + 1], c.c1[0], c.c1[1], c.c1[kPitch],
+                        c.c1[kPitch + 1]};
+    return trilinear<EXACT>(v, qx - bx, qy - by, qz - bz);
 }
 
 // sample_face_half (a node sample: doubled coordinates) of field k.
-template <typename T>
+template <bool EXACT, typename T>
 __device__ __forceinline__ float sample_half(const Window& w, int k, const T* __restrict__ g, int sx, int sy, int sz,
                                              int qx2, int qy2, int qz2) {
     qx2 = min(max(qx2, 0), 2 * (sx - 1));
     qy2 = min(max(qy2, 0), 2 * (sy - 1));
     qz2 = min(max(qz2, 0), 2 * (sz - 1));
     const int ix = qx2 >> 1, iy = qy2 >> 1, iz = qz2 >> 1;
-    if (!inside(w, ix, iy, iz)) return sample_face_half(g, sx, sy, sz, qx2, qy2, qz2);
-    const bool hx = qx2 & 1, hy = qy2 & 1, hz = qz2 & 1;
-    const float wt = (hx ? 0.5f : 1.f) * (hy ? 0.5f : 1.f) * (hz ? 0.5f : 1.f);
+    if (!inside(w, ix, iy, iz)) return sample_face_half<EXACT>(g, sx, sy, sz, qx2, qy2, qz2);
     const Corners c = corners(w, k, ix, iy, iz);
-    float v = 0.f;
-    v = v + wt * c.c0[0];
-    if (hx) v = v + wt * c.c0[1];
-    if (hy) {
-        v = v + wt * c.c0[kPitch];
-        if (hx) v = v + wt * c.c0[kPitch + 1];
-    }
-    if (hz) {
-        v = v + wt * c.c1[0];
-        if (hx) v = v + wt * c.c1[1];
-        if (hy) {
-            v = v + wt * c.c1[kPitch];
-            if (hx) v = v + wt * c.c1[kPitch + 1];
-        }
-    }
-    return v;
+    return half_sample<EXACT>(qx2 & 1, qy2 & 1, qz2 & 1,
+                              [&](int x, int y, int z) { return (z ? c.c1 : c.c0)[y * kPitch + x]; });
 }
 
 }  // namespace tile
@@ -139,11 +114,12 @@ __device__ __forceinline__ int floor_int(float v) {
     return (int)fmaxf(fminf(floorf(v), 1.0e9f), -1.0e9f);
 }
 
-// sample_closed split in two for several scalars sampled at one point: the
+// Closed scalar sample (closed_sample.glsl:7-29), split in two for several
+// scalars sampled at one point: the
 // stencil (clamped corners, fractions and, with colliders, which corners are
 // fluid and the sum of their weights) is formed once, then applied to each
-// field with sample_closed's operations in its order, so every channel's
-// value is sample_closed's.
+// field. Where every corner is fluid (the weights sum to 1) the value is the
+// interpolation; beside a collider, the mean of the fluid corners by weight.
 struct ClosedStencil {
     int rows[4];          // cidx(0, y, z) of (y0, z0), (y1, z0), (y0, z1), (y1, z1)
     int x0, x1;
@@ -171,13 +147,15 @@ __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint
     S.rows[1] = cidx(d, 0, y1, z0);
     S.rows[2] = cidx(d, 0, y0, z1);
     S.rows[3] = cidx(d, 0, y1, z1);
-    S.fluid = 0u;
-    S.total = 0.f;
-    if (MASK) {
+    S.fluid = 255u;
+    S.total = 1.f;
+    if (MASK && !fluid) {
+        S.fluid = 0u;
+        S.total = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int c = S.rows[k >> 1] + ((k & 1) ? S.x1 : S.x0);
-            if (!fluid && __ldg(solid + c)) continue;
+            if (__ldg(solid + c)) continue;
             const float wz = (k & 4) ? S.fz : 1.f - S.fz, wy = (k & 2) ? S.fy : 1.f - S.fy,
                         wx = (k & 1) ? S.fx : 1.f - S.fx;
             S.fluid |= 1u << k;
@@ -189,7 +167,7 @@ __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint
 
 template <typename T, bool MASK>
 __device__ __forceinline__ float apply_closed(const ClosedStencil& S, const T* __restrict__ f) {
-    if (MASK) {
+    if (MASK && S.fluid != 255u) {
         float value = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -200,16 +178,11 @@ __device__ __forceinline__ float apply_closed(const ClosedStencil& S, const T* _
         }
         return S.total > 1e-8f ? value / S.total : 0.f;
     }
-    float f000 = Store<T>::ld(f, S.rows[0] + S.x0), f100 = Store<T>::ld(f, S.rows[0] + S.x1);
-    float f010 = Store<T>::ld(f, S.rows[1] + S.x0), f110 = Store<T>::ld(f, S.rows[1] + S.x1);
-    float f001 = Store<T>::ld(f, S.rows[2] + S.x0), f101 = Store<T>::ld(f, S.rows[2] + S.x1);
-    float f011 = Store<T>::ld(f, S.rows[3] + S.x0), f111 = Store<T>::ld(f, S.rows[3] + S.x1);
-    const float fx = S.fx, fy = S.fy, fz = S.fz;
-    float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    float a0 = f000 * gx + f100 * fx, a1 = f010 * gx + f110 * fx;
-    float b0 = f001 * gx + f101 * fx, b1 = f011 * gx + f111 * fx;
-    float zz0 = a0 * gy + a1 * fy, zz1 = b0 * gy + b1 * fy;
-    return zz0 * gz + zz1 * fz;
+    const float c[8] = {Store<T>::ld(f, S.rows[0] + S.x0), Store<T>::ld(f, S.rows[0] + S.x1),
+                        Store<T>::ld(f, S.rows[1] + S.x0), Store<T>::ld(f, S.rows[1] + S.x1),
+                        Store<T>::ld(f, S.rows[2] + S.x0), Store<T>::ld(f, S.rows[2] + S.x1),
+                        Store<T>::ld(f, S.rows[3] + S.x0), Store<T>::ld(f, S.rows[3] + S.x1)};
+    return trilinear<false>(c, S.fx, S.fy, S.fz);
 }
 
 // ------------------------------------------------------------------ samplers
@@ -257,46 +230,30 @@ template <class Fields>
 struct GlobalSampler {
     Fields f;
 
+    template <bool EXACT>
     __device__ __forceinline__ float sample(int k, float qx, float qy, float qz) const {
         int sx, sy, sz;
         f.dims(k, sx, sy, sz);
-        return sample_face(f.ptr(k), sx, sy, sz, qx, qy, qz);
+        return sample_face<EXACT>(f.ptr(k), sx, sy, sz, qx, qy, qz);
     }
+    template <bool EXACT>
     __device__ __forceinline__ float half(int k, int qx2, int qy2, int qz2) const {
         int sx, sy, sz;
         f.dims(k, sx, sy, sz);
-        return sample_face_half(f.ptr(k), sx, sy, sz, qx2, qy2, qz2);
+        return sample_face_half<EXACT>(f.ptr(k), sx, sy, sz, qx2, qy2, qz2);
     }
     // sample_face_half of field k at the node whose doubled coordinates have the
     // parities (HX, HY, HZ) and lower corner (ix, iy, iz), for a node where no
     // coordinate is clamped (the corners ix..ix+HX etc. lie in the field): the
-    // same terms in the same order with the same power-of-two weight, with the
-    // parities known when compiling.
-    template <int HX, int HY, int HZ>
+    // same value, with the parities known when compiling.
+    template <bool EXACT, int HX, int HY, int HZ>
     __device__ __forceinline__ float node(int k, int ix, int iy, int iz) const {
         int sx, sy, sz;
         f.dims(k, sx, sy, sz);
         const auto* g = f.ptr(k);
         using E = typename std::remove_cv<typename std::remove_pointer<decltype(g)>::type>::type;
-        constexpr float w = (HX ? 0.5f : 1.f) * (HY ? 0.5f : 1.f) * (HZ ? 0.5f : 1.f);
-        const int sxy = sx * sy;
-        const int b = iz * sxy + iy * sx + ix;
-        float v = 0.f;
-        v = v + w * Store<E>::ld(g, b);
-        if (HX) v = v + w * Store<E>::ld(g, b + 1);
-        if (HY) {
-            v = v + w * Store<E>::ld(g, b + sx);
-            if (HX) v = v + w * Store<E>::ld(g, b + sx + 1);
-        }
-        if (HZ) {
-            v = v + w * Store<E>::ld(g, b + sxy);
-            if (HX) v = v + w * Store<E>::ld(g, b + sxy + 1);
-            if (HY) {
-                v = v + w * Store<E>::ld(g, b + sxy + sx);
-                if (HX) v = v + w * Store<E>::ld(g, b + sxy + sx + 1);
-            }
-        }
-        return v;
+        const auto* r = g + (ix + sx * (iy + sy * iz));
+        return half_sample<EXACT>(HX, HY, HZ, [&](int x, int y, int z) { return Store<E>::ld(r, x + sx * (y + sy * z)); });
     }
     // min / max over the eight corners of field k around lower corner (bx, by,
     // bz), each index clamped to the field (correct_velocity_fused.glsl:19-24,
@@ -305,13 +262,19 @@ struct GlobalSampler {
         int sx, sy, sz;
         f.dims(k, sx, sy, sz);
         const auto* g = f.ptr(k);
+        using E = typename std::remove_cv<typename std::remove_pointer<decltype(g)>::type>::type;
+        if ((unsigned)bx < (unsigned)(sx - 1) && (unsigned)by < (unsigned)(sy - 1) && (unsigned)bz < (unsigned)(sz - 1)) {
+            float c[8];
+            load_cube(g, sx, sy, sz, bx + sx * (by + sy * bz), c);
+            cube_range(c, lo, hi);
+            return;
+        }
         const int cx0 = min(max(bx, 0), sx - 1), cx1 = min(max(bx + 1, 0), sx - 1);
         const int cy0 = min(max(by, 0), sy - 1), cy1 = min(max(by + 1, 0), sy - 1);
         const int cz0 = min(max(bz, 0), sz - 1), cz1 = min(max(bz + 1, 0), sz - 1);
         const int sxy = sx * sy;
         const int r0 = cz0 * sxy + cy0 * sx, r1 = cz0 * sxy + cy1 * sx, r2 = cz1 * sxy + cy0 * sx,
                   r3 = cz1 * sxy + cy1 * sx;
-        using E = typename std::remove_cv<typename std::remove_pointer<decltype(g)>::type>::type;
         const float c[8] = {Store<E>::ld(g, r0 + cx0), Store<E>::ld(g, r0 + cx1), Store<E>::ld(g, r1 + cx0),
                             Store<E>::ld(g, r1 + cx1), Store<E>::ld(g, r2 + cx0), Store<E>::ld(g, r2 + cx1),
                             Store<E>::ld(g, r3 + cx0), Store<E>::ld(g, r3 + cx1)};
@@ -346,19 +309,21 @@ struct TileSampler {
     GlobalSampler<Fields> G;
     tile::Window w;
 
+    template <bool EXACT>
     __device__ __forceinline__ float sample(int k, float qx, float qy, float qz) const {
         int sx, sy, sz;
         G.f.dims(k, sx, sy, sz);
-        return tile::sample(w, k, G.f.ptr(k), sx, sy, sz, qx, qy, qz);
+        return tile::sample<EXACT>(w, k, G.f.ptr(k), sx, sy, sz, qx, qy, qz);
     }
+    template <bool EXACT>
     __device__ __forceinline__ float half(int k, int qx2, int qy2, int qz2) const {
         int sx, sy, sz;
         G.f.dims(k, sx, sy, sz);
-        return tile::sample_half(w, k, G.f.ptr(k), sx, sy, sz, qx2, qy2, qz2);
+        return tile::sample_half<EXACT>(w, k, G.f.ptr(k), sx, sy, sz, qx2, qy2, qz2);
     }
-    template <int HX, int HY, int HZ>
+    template <bool EXACT, int HX, int HY, int HZ>
     __device__ __forceinline__ float node(int k, int ix, int iy, int iz) const {
-        return G.template node<HX, HY, HZ>(k, ix, iy, iz);
+        return G.template node<EXACT, HX, HY, HZ>(k, ix, iy, iz);
     }
     __device__ __forceinline__ void minmax8(int k, int bx, int by, int bz, float& lo, float& hi) const {
         // the window holds clamp(index) at every entry, so the clamped corners
@@ -412,7 +377,7 @@ struct TileSampler {
             const float* r = (j & 4) ? c1 : c0;
             return r[((j & 2) ? tile::kPitch : 0) + (j & 1)];
         };
-        if (MASK) {
+        if (MASK && S.fluid != 255u) {
             float value = 0.f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -423,67 +388,83 @@ struct TileSampler {
             }
             return S.total > 1e-8f ? value / S.total : 0.f;
         }
-        const float f000 = corner(0), f100 = corner(1), f010 = corner(2), f110 = corner(3);
-        const float f001 = corner(4), f101 = corner(5), f011 = corner(6), f111 = corner(7);
-        const float fx = S.fx, fy = S.fy, fz = S.fz;
-        const float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-        const float a0 = f000 * gx + f100 * fx, a1 = f010 * gx + f110 * fx;
-        const float b0 = f001 * gx + f101 * fx, b1 = f011 * gx + f111 * fx;
-        const float zz0 = a0 * gy + a1 * fy, zz1 = b0 * gy + b1 * fy;
-        return zz0 * gz + zz1 * fz;
+        const float c[8] = {corner(0), corner(1), corner(2), corner(3), corner(4), corner(5), corner(6), corner(7)};
+        return trilinear<false>(c, S.fx, S.fy, S.fz);
     }
 };
 
+// Grid coordinate of a traced position along axis i.
+template <bool MASK, bool P2>
+__device__ __forceinline__ float cells(const Dev& d, float x, int i) {
+    return !MASK && !P2 ? x * d.rc[i] : dv_h<P2>(d, x, i);
+}
+
 // Staggered velocity at a physical point through a sampler (velocity_at).
-template <bool P2, class S>
+template <bool MASK, bool P2, class S>
 __device__ __forceinline__ F3 velocity_s(const Dev& d, const S& smp, F3 p) {
-    const float qx = dv_e<P2>(d, p.x * d.nf[0], 0);
-    const float qy = dv_e<P2>(d, p.y * d.nf[1], 1);
-    const float qz = dv_e<P2>(d, p.z * d.nf[2], 2);
+    float q[3];
+    const float pp[3] = {p.x, p.y, p.z};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if (MASK && !P2)      // beyond 2^96 (or not a number) the sample's clamp decides
+            q[i] = div_near(fminf(fmaxf(pp[i] * d.nf[i], -0x1p96f), 0x1p96f), d.e[i], d.re[i]);
+        else
+            q[i] = pp[i] * d.rc[i];
+    }
     F3 r;
-    r.x = smp.sample(0, qx, qy - 0.5f, qz - 0.5f);
-    r.y = smp.sample(1, qx - 0.5f, qy, qz - 0.5f);
-    r.z = smp.sample(2, qx - 0.5f, qy - 0.5f, qz);
+    r.x = smp.template sample<MASK>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
+    r.y = smp.template sample<MASK>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
+    r.z = smp.template sample<MASK>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
     return r;
 }
 
-// Velocity at the node p = (X2, Y2, Z2) / 2 cells (velocity_at_start).
-template <bool P2, class S>
+// Velocity at the face centre p = (X2, Y2, Z2) / 2 cells.
+template <bool MASK, bool P2, class S>
 __device__ __forceinline__ F3 start_velocity_s(const Dev& d, const S& smp, F3 p, int X2, int Y2, int Z2) {
-    if constexpr (P2) {
+    if constexpr (!MASK || P2) {
         F3 r;
-        r.x = smp.half(0, X2, Y2 - 1, Z2 - 1);
-        r.y = smp.half(1, X2 - 1, Y2, Z2 - 1);
-        r.z = smp.half(2, X2 - 1, Y2 - 1, Z2);
+        r.x = smp.template half<MASK>(0, X2, Y2 - 1, Z2 - 1);
+        r.y = smp.template half<MASK>(1, X2 - 1, Y2, Z2 - 1);
+        r.z = smp.template half<MASK>(2, X2 - 1, Y2 - 1, Z2);
         return r;
     } else {
-        return velocity_s<false>(d, smp, p);
+        return velocity_s<true, false>(d, smp, p);
     }
 }
 
+// Velocity at the centre p of cell (x, y, z): the two faces along each axis.
+template <bool MASK, bool P2, class S>
+__device__ __forceinline__ F3 start_velocity_cell(const Dev& d, const S& smp, F3 p, int x, int y, int z) {
+    if constexpr (!MASK || P2)
+        return F3{smp.template node<MASK, 1, 0, 0>(0, x, y, z), smp.template node<MASK, 0, 1, 0>(1, x, y, z),
+                  smp.template node<MASK, 0, 0, 1>(2, x, y, z)};
+    else
+        return velocity_s<true, false>(d, smp, p);
+}
+
 // Velocity at the centre p of face (x, y, z) of face grid `axis`
-// (start_velocity_s at its doubled coordinates). On power-of-two grids, for a
+// (start_velocity_s at its doubled coordinates). Where those are used, for a
 // face off the domain walls along its axis, no doubled coordinate is clamped
 // and the parities of every component's node are fixed by the axis: the U face
 // (2x, 2y+1, 2z+1) reads u at (x, y, z), v at (x-1..x, y..y+1, z) and w at
 // (x-1..x, y, z..z+1), and likewise for V and W faces.
-template <bool P2, class S>
+template <bool MASK, bool P2, class S>
 __device__ __forceinline__ F3 start_velocity_face(const Dev& d, const S& smp, F3 p, int axis, int x, int y, int z) {
-    if constexpr (P2) {
+    if constexpr (!MASK || P2) {
         const int c = axis == 0 ? x : (axis == 1 ? y : z);
         const int n = axis == 0 ? d.nx : (axis == 1 ? d.ny : d.nz);
         if (c >= 1 && c <= n - 1) {
             if (axis == 0)
-                return F3{smp.template node<0, 0, 0>(0, x, y, z), smp.template node<1, 1, 0>(1, x - 1, y, z),
-                          smp.template node<1, 0, 1>(2, x - 1, y, z)};
+                return F3{smp.template node<MASK, 0, 0, 0>(0, x, y, z), smp.template node<MASK, 1, 1, 0>(1, x - 1, y, z),
+                          smp.template node<MASK, 1, 0, 1>(2, x - 1, y, z)};
             if (axis == 1)
-                return F3{smp.template node<1, 1, 0>(0, x, y - 1, z), smp.template node<0, 0, 0>(1, x, y, z),
-                          smp.template node<0, 1, 1>(2, x, y - 1, z)};
-            return F3{smp.template node<1, 0, 1>(0, x, y, z - 1), smp.template node<0, 1, 1>(1, x, y, z - 1),
-                      smp.template node<0, 0, 0>(2, x, y, z)};
+                return F3{smp.template node<MASK, 1, 1, 0>(0, x, y - 1, z), smp.template node<MASK, 0, 0, 0>(1, x, y, z),
+                          smp.template node<MASK, 0, 1, 1>(2, x, y - 1, z)};
+            return F3{smp.template node<MASK, 1, 0, 1>(0, x, y, z - 1), smp.template node<MASK, 0, 1, 1>(1, x, y, z - 1),
+                      smp.template node<MASK, 0, 0, 0>(2, x, y, z)};
         }
     }
-    return start_velocity_s<P2>(d, smp, p, 2 * x + (axis != 0), 2 * y + (axis != 1), 2 * z + (axis != 2));
+    return start_velocity_s<MASK, P2>(d, smp, p, 2 * x + (axis != 0), 2 * y + (axis != 1), 2 * z + (axis != 2));
 }
 
 // Midpoint backtrace through a sampler (the `backtrace` of the transport
@@ -494,7 +475,7 @@ __device__ __forceinline__ F3 backtrace_s(const Dev& d, const S& smp, const uint
     const float s = 0.5f * dt;
     F3 mid = {p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z};
     if (MASK) mid = clip_from<P2>(d, solid, halo, cv, p, mid);
-    const F3 vm = velocity_s<P2>(d, smp, mid);
+    const F3 vm = velocity_s<MASK, P2>(d, smp, mid);
     F3 dep = {p.x - dt * vm.x, p.y - dt * vm.y, p.z - dt * vm.z};
     if (MASK) dep = clip_from<P2>(d, solid, halo, cv, p, dep);
     return dep;
