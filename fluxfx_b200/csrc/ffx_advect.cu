@@ -1326,34 +1326,39 @@ struct DeviceDt {
     __device__ __forceinline__ void operator()(D& sh, int slot) const { sh.dt = sign * state[slot].dt; }
 };
 
+// P2: every domain of the launch has powers of two for its e, n and h. A mixed
+// launch takes the general form for all: its quotients are exact for those
+// domains too, and one form in the kernel instead of both spares the registers
+// (velocity: 312 bytes of stack and 1100 of spills with both).
+template <bool P2>
 __global__ void FFX_LB_BATCH_PREDICTOR batch_predictor_kernel(const __grid_constant__ BatchMap M,
                                                                         const PredParams<float>* descs,
                                                                         const BatchState* state) {
     for_tiles(M, descs, state, false, DeviceDt{state, 1.f}, [](const PredParams<float>& P, const Blk& b, int) {
-        if (P.d.pow2) face_predictor_body<float, true, true>(P, b);
-        else face_predictor_body<float, true, false>(P, b);
+        face_predictor_body<float, true, P2>(P, b);
     });
 }
 
+template <bool P2>
 __global__ void FFX_LB_BATCH_VELOCITY batch_velocity_kernel(const __grid_constant__ BatchMap M,
                                                                        const VelParams<float>* descs,
                                                                        const BatchState* state) {
     for_tiles(M, descs, state, false, DeviceDt{state, 1.f}, [](const VelParams<float>& P, const Blk& b, int) {
-        if (P.d.pow2) advect_velocity_body<float, true, true>(P, b);
-        else advect_velocity_body<float, true, false>(P, b);
+        advect_velocity_body<float, true, P2>(P, b);
     });
 }
 
+template <bool P2>
 __global__ void __launch_bounds__(kBatchThreads) batch_scalar_transport_kernel(const __grid_constant__ BatchMap M,
                                                                                const ScalarXport<float>* descs,
                                                                                const BatchState* state, float sign) {
     for_tiles(M, descs, state, false, DeviceDt{state, sign}, [](const ScalarXport<float>& P, const Blk& b, int) {
-        if (P.d.pow2) scalar_transport_body<float, true, true>(P, b);
-        else scalar_transport_body<float, true, false>(P, b);
+        scalar_transport_body<float, true, P2>(P, b);
     });
 }
 
 // The reverse pass: domains with decision buffers decide the final pass's corrections.
+template <bool P2>
 __global__ void __launch_bounds__(kBatchThreads) batch_scalar_reverse_kernel(const __grid_constant__ BatchMap M,
                                                                              const ScalarXport<float>* descs,
                                                                              const BatchState* state) {
@@ -1363,21 +1368,19 @@ __global__ void __launch_bounds__(kBatchThreads) batch_scalar_reverse_kernel(con
         if (!cell_coords(b, P.d.nx, P.d.ny, x, y, z)) return;
         const auto smp = cell_sampler<float>(P.d, P.F, P.in);
         if (P.ok) {
-            if (P.d.pow2) scalar_transport_cell<float, true, true, S, true>(P, x, y, z, smp);
-            else scalar_transport_cell<float, true, false, S, true>(P, x, y, z, smp);
+            scalar_transport_cell<float, true, P2, S, true>(P, x, y, z, smp);
         } else {
-            if (P.d.pow2) scalar_transport_cell<float, true, true, S, false>(P, x, y, z, smp);
-            else scalar_transport_cell<float, true, false, S, false>(P, x, y, z, smp);
+            scalar_transport_cell<float, true, P2, S, false>(P, x, y, z, smp);
         }
     });
 }
 
+template <bool P2>
 __global__ void FFX_LB_BATCH_SCALARS batch_scalars_kernel(const __grid_constant__ BatchMap M,
                                                                       const ScalarFinal<float>* descs,
                                                                       const BatchState* state) {
     for_tiles(M, descs, state, false, DeviceDt{state, 1.f}, [](const ScalarFinal<float>& P, const Blk& b, int) {
-        if (P.d.pow2) advect_scalars_body<float, true, true>(P, b);
-        else advect_scalars_body<float, true, false>(P, b);
+        advect_scalars_body<float, true, P2>(P, b);
     });
 }
 
@@ -1515,35 +1518,35 @@ size_t scalar_final_desc(const FfxBatchDomain& D, int parity, void* out) {
 }
 
 cudaError_t face_predictor(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    batch_predictor_kernel<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const PredParams<float>*)descs, state);
+    (M.pow2 ? batch_predictor_kernel<true> : batch_predictor_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const PredParams<float>*)descs, state);
     return cudaGetLastError();
 }
 cudaError_t advect_velocity(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    batch_velocity_kernel<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const VelParams<float>*)descs, state);
+    (M.pow2 ? batch_velocity_kernel<true> : batch_velocity_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const VelParams<float>*)descs, state);
     return cudaGetLastError();
 }
 cudaError_t scalar_transport(const BatchMap& M, const void* descs, BatchState* state, int reverse, int grid,
                              cudaStream_t st) {
     if (reverse)
-        batch_scalar_reverse_kernel<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarXport<float>*)descs,
+        (M.pow2 ? batch_scalar_reverse_kernel<true> : batch_scalar_reverse_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarXport<float>*)descs,
                                                                                state);
     else
-        batch_scalar_transport_kernel<<<grid_of(M, grid), kBatchThreads, 0, st>>>(
+        (M.pow2 ? batch_scalar_transport_kernel<true> : batch_scalar_transport_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(
             M, (const ScalarXport<float>*)descs, state, 1.f);
     return cudaGetLastError();
 }
 cudaError_t advect_scalars(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    batch_scalars_kernel<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarFinal<float>*)descs, state);
+    (M.pow2 ? batch_scalars_kernel<true> : batch_scalars_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarFinal<float>*)descs, state);
     return cudaGetLastError();
 }
 
 int advect_resident_blocks(int kind) {
     switch (kind) {
-        case kPredictor: return occupancy(batch_predictor_kernel);
-        case kVelocity: return occupancy(batch_velocity_kernel);
+        case kPredictor: return occupancy(batch_predictor_kernel<false>);
+        case kVelocity: return occupancy(batch_velocity_kernel<false>);
         case kScalarPredictor:
-        case kScalarReverse: return occupancy(batch_scalar_reverse_kernel);
-        case kScalarFinal: return occupancy(batch_scalars_kernel);
+        case kScalarReverse: return occupancy(batch_scalar_reverse_kernel<false>);
+        case kScalarFinal: return occupancy(batch_scalars_kernel<false>);
         default: return 0;
     }
 }

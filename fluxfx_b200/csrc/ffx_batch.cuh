@@ -24,6 +24,7 @@ constexpr int kBatchZ0 = 8;         // z cells per thread of the level-0 sweeps
 struct BatchMap {
     int count;                // entries (domains) in this launch
     int total;                // tiles over all entries
+    int pow2;                 // every entry's e, n and h are powers of two
     int bw, bh;               // tile shape: bw x bh threads (bw * bh == kBatchThreads)
     int dom[kBatchMax];       // state slot of entry k
     int first[kBatchMax + 1]; // first tile of entry k; first[count] == total
