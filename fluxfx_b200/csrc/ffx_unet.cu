@@ -32,7 +32,8 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kBM = 128, kBN = 64, kStages = 3, kGemmThreads = 128;
+constexpr int kBM = 128, kBN = 64, kGemmThreads = 128;
+constexpr int kFwdStages = 5;   // ring of the forward GEMM: 42 KB at BN = 64
 constexpr int kAStride = 24;    // bf16 per A row in shared memory (16 + 8 pad: 48 B, conflict-free ldmatrix)
 constexpr int kBStride = 72;    // bf16 per B row (64 + 8 pad: 144 B)
 
@@ -126,6 +127,39 @@ __device__ __forceinline__ const bf16* gather(const Conv& a, const RowPos& pos, 
     return a.in2.p + vox * a.in2.pitch + a.in2.offset + (c - a.c1);
 }
 
+// The units (8 channels each) of GEMM row `pos` one after another, tap by tap:
+// the address of the next, or nullptr where its tap falls outside the input
+// (zero padding). The tap's voxel is found once per tap.
+struct UnitWalk {
+    RowPos pos;
+    int tap, c;
+    long long vox;      // < 0: outside
+    __device__ __forceinline__ UnitWalk(const Conv& a, RowPos p) : pos(p), tap(0), c(0) { place(a); }
+    __device__ __forceinline__ void place(const Conv& a) {
+        if (a.transposed) {
+            vox = (((long long)pos.b * a.id + pos.z) * a.ih + pos.y) * a.iw + pos.x;
+            return;
+        }
+        const int ks = a.ks, dz = tap / (ks * ks), r = tap - dz * ks * ks, dy = r / ks, dx = r - dy * ks;
+        const int zz = pos.z * a.stride - a.pad + dz, yy = pos.y * a.stride - a.pad + dy,
+                  xx = pos.x * a.stride - a.pad + dx;
+        const bool in = (unsigned)zz < (unsigned)a.id && (unsigned)yy < (unsigned)a.ih && (unsigned)xx < (unsigned)a.iw;
+        vox = in ? (((long long)pos.b * a.id + zz) * a.ih + yy) * a.iw + xx : -1;
+    }
+    __device__ __forceinline__ const bf16* next(const Conv& a) {
+        const bf16* at = vox < 0 ? nullptr
+                         : c < a.c1 ? a.in1.p + vox * a.in1.pitch + a.in1.offset + c
+                                    : a.in2.p + vox * a.in2.pitch + a.in2.offset + (c - a.c1);
+        c += 8;
+        if (c == 8 * a.units_per_tap) {
+            c = 0;
+            ++tap;
+            place(a);
+        }
+        return at;
+    }
+};
+
 // Output voxel index of GEMM row m (class j for the transposed form).
 __device__ __forceinline__ long long out_voxel(const Conv& a, long long m, int cls) {
     if (!a.transposed) return m;
@@ -136,12 +170,19 @@ __device__ __forceinline__ long long out_voxel(const Conv& a, long long m, int c
 
 // ------------------------------------------------------------ forward GEMM
 // BN output channels per block (16, 32 or 64, chosen from cout so that narrow
-// layers do not multiply padded channels).
+// layers do not multiply padded channels, halved while the grid would leave SMs
+// without a block).
+//
+// Bound by the latency of a k-step: the layers that come here have a few hundred
+// to a few thousand rows and 8 to 64 steps. The rows' addresses are walked tap by
+// tap instead of divided out per unit, and four steps are in flight. With two
+// steps in flight and 64 channels a block whatever the grid, the five layers of a
+// guess at 128 x 96 x 64 took 118 us, now 79.
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads) conv_fwd_kernel(const __grid_constant__ Conv a) {
     constexpr int BS = BN + 8;   // bf16 per B row in shared memory (8 pad: conflict-free ldmatrix)
-    __shared__ __align__(128) bf16 sA[kStages][kBM * kAStride];
-    __shared__ __align__(128) bf16 sB[kStages][16 * BS];
+    __shared__ __align__(128) bf16 sA[kFwdStages][kBM * kAStride];
+    __shared__ __align__(128) bf16 sB[kFwdStages][16 * BS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long m0 = (long long)blockIdx.x * kBM;
     const int n0 = blockIdx.y * BN;
@@ -154,11 +195,12 @@ __global__ void __launch_bounds__(kGemmThreads) conv_fwd_kernel(const __grid_con
     const int k_elems = a.k_units * 8;
     const int nk = (a.k_units + 1) / 2;
 
-    auto load = [&](int stage, int kstep) {
+    UnitWalk walk(a, pos);
+    auto load = [&](int stage, int kstep) {      // steps in order
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int u = kstep * 2 + h;
-            const bf16* src = (row_ok && u < a.k_units) ? gather(a, pos, u) : nullptr;
+            const bf16* src = (row_ok && u < a.k_units) ? walk.next(a) : nullptr;
             cp_async16(&sA[stage][tid * kAStride + h * 8], src ? src : a.in1.p, src != nullptr);
         }
         if (tid < 2 * BN) {   // 16 rows x BN / 8 units of 8 channels
@@ -178,17 +220,17 @@ __global__ void __launch_bounds__(kGemmThreads) conv_fwd_kernel(const __grid_con
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
 
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
+    for (int s = 0; s < kFwdStages - 1; ++s) {
         if (s < nk) load(s, s);
         cp_async_commit();
     }
     for (int ks = 0; ks < nk; ++ks) {
-        cp_async_wait<kStages - 2>();
+        cp_async_wait<kFwdStages - 2>();
         __syncthreads();
-        const int pf = ks + kStages - 1;
-        if (pf < nk) load(pf % kStages, pf);
+        const int pf = ks + kFwdStages - 1;
+        if (pf < nk) load(pf % kFwdStages, pf);
         cp_async_commit();
-        const int st = ks % kStages;
+        const int st = ks % kFwdStages;
         unsigned af[2][4];
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)
@@ -785,48 +827,15 @@ __global__ void __launch_bounds__(kTmThreads, 1) conv3_tma_kernel(const __grid_c
 // 1^3 convolutions and transposed 2^3 stride-2 convolutions with 8 or 16
 // output channels: each output voxel is one dot product of its input (parent)
 // voxel's channels with the weights of its tap, and a tensor-core tile of 128
-// voxels x 16 channels would be mostly idle. A thread computes one output
-// voxel: the input channels in 16-byte groups, the weights of all taps as FP32
-// in shared memory, FP32 fused multiply-adds in channel order, then the bias,
-// ReLU, accumulation and BF16 / FP32 stores of the implicit-GEMM epilogue.
+// voxels x 16 channels would be mostly idle. The input channels come in 16-byte
+// groups, the weights as FP32 from shared memory; FP32 fused multiply-adds in
+// channel order (two output channels to an instruction), then the bias, ReLU,
+// accumulation and BF16 / FP32 stores of the implicit-GEMM epilogue.
 constexpr int kDirectThreads = 256;
 constexpr int kDirectMaxWeights = 12288;   // taps x cin x cout FP32 values (48 KB)
 
 template <int COUT>
-__global__ void __launch_bounds__(kDirectThreads) conv_direct_kernel(const __grid_constant__ Conv a) {
-    extern __shared__ float ws[];          // [taps][cin][COUT]
-    const int taps = a.transposed ? 8 : 1;
-    const int nw = taps * a.cin * COUT;
-    for (int i = threadIdx.x; i < nw; i += kDirectThreads) ws[i] = __bfloat162float(a.w[i]);
-    __syncthreads();
-    const long long o = (long long)blockIdx.x * kDirectThreads + threadIdx.x;
-    if (o >= (long long)a.batch * a.od * a.oh * a.ow) return;
-    const RowPos p = decode(o, a.od, a.oh, a.ow);
-    int tap = 0;
-    long long q = o;
-    if (a.transposed) {
-        // output voxel 2 q + j is tap j of input voxel q
-        tap = ((p.z & 1) << 2) | ((p.y & 1) << 1) | (p.x & 1);
-        q = (((long long)p.b * a.id + (p.z >> 1)) * a.ih + (p.y >> 1)) * a.iw + (p.x >> 1);
-    }
-    const float* W = ws + tap * a.cin * COUT;
-    const bf16* x = a.in1.p + q * a.in1.pitch + a.in1.offset;
-    float acc[COUT];
-#pragma unroll
-    for (int n = 0; n < COUT; ++n) acc[n] = 0.f;
-    for (int c8 = 0; c8 < a.cin; c8 += 8) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(x + c8);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __bfloat1622float2(h[e]);
-            const float* w0 = W + (c8 + 2 * e) * COUT;
-#pragma unroll
-            for (int n = 0; n < COUT; ++n) acc[n] = __fmaf_rn(f.x, w0[n], acc[n]);
-#pragma unroll
-            for (int n = 0; n < COUT; ++n) acc[n] = __fmaf_rn(f.y, w0[COUT + n], acc[n]);
-        }
-    }
+__device__ __forceinline__ void store_direct(const Conv& a, long long o, float (&acc)[COUT]) {
 #pragma unroll
     for (int n = 0; n < COUT; ++n) {
         if (a.bias) acc[n] += __ldg(a.bias + n);
@@ -858,6 +867,84 @@ __global__ void __launch_bounds__(kDirectThreads) conv_direct_kernel(const __gri
 #pragma unroll
         for (int n = 0; n < COUT; ++n) dst[n] = acc[n];
     }
+}
+
+// acc[pair] += x w[pair] over the channels of one voxel for NT taps whose weights
+// lie `step` floats apart.
+template <int COUT, int NT>
+__device__ __forceinline__ void dot_direct(const bf16* x, int cin, const float* W, int step, float (&out)[NT][COUT]) {
+    unsigned long long acc[NT][COUT / 2];
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int n = 0; n < COUT / 2; ++n) acc[t][n] = 0ull;
+    for (int c8 = 0; c8 < cin; c8 += 8) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(x + c8);
+        const unsigned h[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const unsigned bits = e & 1 ? h[e / 2] & 0xffff0000u : h[e / 2] << 16;      // BF16 -> FP32
+            const unsigned long long f = (unsigned long long)bits << 32 | bits;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const ulonglong2* w = reinterpret_cast<const ulonglong2*>(W + t * step + (c8 + e) * COUT);
+#pragma unroll
+                for (int n = 0; n < COUT / 4; ++n) {
+                    const ulonglong2 v = w[n];
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][2 * n]) : "l"(f), "l"(v.x));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][2 * n + 1]) : "l"(f), "l"(v.y));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int n = 0; n < COUT / 2; ++n) {
+            out[t][2 * n] = __uint_as_float((unsigned)acc[t][n]);
+            out[t][2 * n + 1] = __uint_as_float((unsigned)(acc[t][n] >> 32));
+        }
+}
+
+// 1^3: a thread per voxel.
+template <int COUT>
+__global__ void __launch_bounds__(kDirectThreads) conv_direct_kernel(const __grid_constant__ Conv a) {
+    extern __shared__ __align__(16) float ws[];          // [cin][COUT]
+    for (int i = threadIdx.x; i < a.cin * COUT; i += kDirectThreads) ws[i] = __bfloat162float(a.w[i]);
+    __syncthreads();
+    const long long o = (long long)blockIdx.x * kDirectThreads + threadIdx.x;
+    if (o >= (long long)a.batch * a.od * a.oh * a.ow) return;
+    float acc[1][COUT];
+    dot_direct<COUT, 1>(a.in1.p + o * a.in1.pitch + a.in1.offset, a.cin, ws, 0, acc);
+    store_direct<COUT>(a, o, acc[0]);
+}
+
+// Transposed: a thread per input voxel and (z, y) tap, the output voxels of both
+// x taps; blockIdx.y is the (z, y) tap, so a block's threads read the same
+// weights (one shared-memory word for a warp) and each input value serves two
+// outputs. A thread per output voxel, its tap by its parity, was bound by those
+// reads: 32 -> 16 channels at 128 x 96 x 64 59 us, now 40.
+template <int COUT>
+__global__ void __launch_bounds__(kDirectThreads) conv_up_kernel(const __grid_constant__ Conv a) {
+    extern __shared__ __align__(16) float ws[];          // [2][cin][COUT]
+    const int zy = blockIdx.y, step = a.cin * COUT;
+    const bf16* w = a.w + (size_t)(2 * zy) * step;
+    for (int i = threadIdx.x; i < 2 * step; i += kDirectThreads) ws[i] = __bfloat162float(w[i]);
+    __syncthreads();
+    const long long q = (long long)blockIdx.x * kDirectThreads + threadIdx.x;
+    if (q >= a.rows) return;
+    RowPos p;
+    if (a.rows < (1ll << 31)) {
+        const unsigned m = (unsigned)q, w1 = m / (unsigned)a.iw, h1 = w1 / (unsigned)a.ih, d1 = h1 / (unsigned)a.id;
+        p = RowPos{(int)d1, (int)(h1 - d1 * a.id), (int)(w1 - h1 * a.ih), (int)(m - w1 * a.iw)};
+    } else {
+        p = decode(q, a.id, a.ih, a.iw);
+    }
+    float acc[2][COUT];
+    dot_direct<COUT, 2>(a.in1.p + q * a.in1.pitch + a.in1.offset, a.cin, ws, step, acc);
+    const long long o = (((long long)p.b * a.od + 2 * p.z + (zy >> 1)) * a.oh + 2 * p.y + (zy & 1)) * a.ow + 2 * p.x;
+    store_direct<COUT>(a, o, acc[0]);
+    store_direct<COUT>(a, o + 1, acc[1]);
 }
 
 // Packed weights of the TMA convolution: w[k = tap * cin + c][cout] ->
@@ -1413,7 +1500,9 @@ int ffx_conv_forward(const FfxConv* c, void* stream) {
     int e = make_conv(c, a);
     if (e) return e;
     FFX_REQUIRE(a.out || a.out_f32, "ffx_conv_forward: no output");
-    const int bn = a.cout <= 16 ? 16 : (a.cout <= 32 ? 32 : 64);
+    int bn = a.cout <= 16 ? 16 : (a.cout <= 32 ? 32 : 64);
+    const long long row_blocks = (a.rows + kBM - 1) / kBM * (a.transposed ? 8 : 1);
+    while (bn > 16 && row_blocks * ((a.cout + bn - 1) / bn) < sm_count()) bn /= 2;
     const dim3 grid((unsigned)((a.rows + kBM - 1) / kBM), (unsigned)((a.cout + bn - 1) / bn), a.transposed ? 8 : 1);
     FFX_REQUIRE(grid.x < (1u << 31), "ffx_conv_forward: grid too large");
     if (bn == 16) conv_fwd_kernel<16><<<grid, kGemmThreads, 0, as_stream(stream)>>>(a);
@@ -1476,7 +1565,14 @@ int ffx_conv_forward_tma(const FfxConv* c, const void* packed, void* stream) {
         if ((one || a.transposed) && (a.cout == 8 || a.cout == 16) && a.c2 == 0 &&
             (a.transposed ? 8 : 1) * a.cin * a.cout <= kDirectMaxWeights && (a.out || a.out_f32)) {
             const long long vox = (long long)a.batch * a.od * a.oh * a.ow;
-            const size_t smem = sizeof(float) * (size_t)(a.transposed ? 8 : 1) * a.cin * a.cout;
+            if (a.transposed) {
+                const size_t smem = sizeof(float) * 2 * (size_t)a.cin * a.cout;
+                const dim3 grid((unsigned)((a.rows + kDirectThreads - 1) / kDirectThreads), 4);
+                if (a.cout == 8) conv_up_kernel<8><<<grid, kDirectThreads, smem, as_stream(stream)>>>(a);
+                else conv_up_kernel<16><<<grid, kDirectThreads, smem, as_stream(stream)>>>(a);
+                return launch_status("conv_up_kernel");
+            }
+            const size_t smem = sizeof(float) * (size_t)a.cin * a.cout;
             const unsigned blocks = (unsigned)((vox + kDirectThreads - 1) / kDirectThreads);
             if (a.cout == 8) conv_direct_kernel<8><<<blocks, kDirectThreads, smem, as_stream(stream)>>>(a);
             else conv_direct_kernel<16><<<blocks, kDirectThreads, smem, as_stream(stream)>>>(a);
