@@ -165,10 +165,10 @@ __device__ __forceinline__ void face_predictor_axis(const PredParams<T>& P, Face
     }
     float ox = f.axis == 0 ? 0.f : 0.5f, oy = f.axis == 1 ? 0.f : 0.5f, oz = f.axis == 2 ? 0.f : 0.5f;
     F3 p = {((float)f.x + ox) * d.h[0], ((float)f.y + oy) * d.h[1], ((float)f.z + oz) * d.h[2]};
-    F3 v0 = start_velocity_face<MASK, P2>(d, smp, p, f.axis, f.x, f.y, f.z);
-    F3 dep = backtrace_s<MASK, P2>(d, smp, solid, halo, p, v0, dt, cv);
-    float value = smp.template sample<MASK>(f.axis, cells<MASK, P2>(d, dep.x, 0) - ox, cells<MASK, P2>(d, dep.y, 1) - oy,
-                             cells<MASK, P2>(d, dep.z, 2) - oz);
+    F3 v0 = start_velocity_face<EXACT<T, MASK>, P2>(d, smp, p, f.axis, f.x, f.y, f.z);
+    F3 dep = backtrace_s<MASK, EXACT<T, MASK>, P2>(d, smp, solid, halo, p, v0, dt, cv);
+    float value = smp.template sample<EXACT<T, MASK>>(f.axis, cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - ox, cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - oy,
+                             cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - oz);
     Store<T>::st(out, f.i, value);
     if (float* D = P.dep[f.axis]) {
         const int nf = P.nf[f.axis];
@@ -262,16 +262,16 @@ __device__ __forceinline__ void advect_velocity_axis(const VelParams<T>& P, Face
             dep = {__ldg(D + f.i), __ldg(D + f.i + nf), __ldg(D + f.i + 2 * nf)};
             v0 = {__ldg(D + f.i + kV0 * nf), __ldg(D + f.i + (kV0 + 1) * nf), __ldg(D + f.i + (kV0 + 2) * nf)};
         } else {
-            v0 = start_velocity_face<MASK, P2>(d, smp, p, axis, f.x, f.y, f.z);
-            dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
+            v0 = start_velocity_face<EXACT<T, MASK>, P2>(d, smp, p, axis, f.x, f.y, f.z);
+            dep = backtrace_s<MASK, EXACT<T, MASK>, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
         }
         const T* orig = axis == 0 ? P.F.u : (axis == 1 ? P.F.v : P.F.w);
         const T* pred = axis == 0 ? P.P.u : (axis == 1 ? P.P.v : P.P.w);
-        float qx = cells<MASK, P2>(d, dep.x, 0) - off[0], qy = cells<MASK, P2>(d, dep.y, 1) - off[1],
-              qz = cells<MASK, P2>(d, dep.z, 2) - off[2];
+        float qx = cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - off[0], qy = cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - off[1],
+              qz = cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - off[2];
         // the predictor's sample at the same departure point: the stored value
         // (FP32) or its unrounded copy in the fourth trace plane (BF16)
-        float low = !reuse ? smp.template sample<MASK>(axis, qx, qy, qz)
+        float low = !reuse ? smp.template sample<EXACT<T, MASK>>(axis, qx, qy, qz)
                            : (sizeof(T) == 4 ? Store<T>::ld(pred, f.i) : __ldg(P.dep[axis] + f.i + 3 * P.nf[axis]));
         value = low;
         if (P.corrected) {
@@ -284,15 +284,15 @@ __device__ __forceinline__ void advect_velocity_axis(const VelParams<T>& P, Face
             }
             float s = 0.5f * dt;
             F3 mid2 = {p.x + s * v0.x, p.y + s * v0.y, p.z + s * v0.z};
-            F3 vm2 = velocity_s<MASK, P2>(d, smp, mid2);
+            F3 vm2 = velocity_s<EXACT<T, MASK>, P2>(d, smp, mid2);
             F3 arr = {p.x + dt * vm2.x, p.y + dt * vm2.y, p.z + dt * vm2.z};
             bool ok = !(dep.x < lob[0] || dep.y < lob[1] || dep.z < lob[2] || dep.x > hib[0] || dep.y > hib[1] ||
                         dep.z > hib[2] || arr.x < lob[0] || arr.y < lob[1] || arr.z < lob[2] || arr.x > hib[0] ||
                         arr.y > hib[1] || arr.z > hib[2]);
             if (MASK && ok) ok = safe_correction_from<P2>(d, P.solid, P.halo, cv, p, dep, mid2, arr);
             if (ok) {
-                float pa = smp.template sample<MASK>(3 + axis, cells<MASK, P2>(d, arr.x, 0) - off[0], cells<MASK, P2>(d, arr.y, 1) - off[1],
-                                      cells<MASK, P2>(d, arr.z, 2) - off[2]);
+                float pa = smp.template sample<EXACT<T, MASK>>(3 + axis, cells<EXACT<T, MASK>, P2>(d, arr.x, 0) - off[0], cells<EXACT<T, MASK>, P2>(d, arr.y, 1) - off[1],
+                                      cells<EXACT<T, MASK>, P2>(d, arr.z, 2) - off[2]);
                 float val = Store<T>::ld(pred, f.i) + 0.5f * (Store<T>::ld(orig, f.i) - pa);
                 // min / max of the 8 corners around the departure point, clamped to the grid
                 float lo, hi;
@@ -574,7 +574,7 @@ __device__ __forceinline__ void scalar_transport_cell(const ScalarXport<T>& P, i
         return;
     }
     F3 p = {((float)x + 0.5f) * d.h[0], ((float)y + 0.5f) * d.h[1], ((float)z + 0.5f) * d.h[2]};
-    F3 v0 = start_velocity_cell<MASK, P2>(d, smp, p, x, y, z);
+    F3 v0 = start_velocity_cell<EXACT<T, MASK>, P2>(d, smp, p, x, y, z);
     F3 dep;
     if (DECIDE) {
         // backtrace_s, keeping the unclipped midpoint and departure point: with
@@ -585,20 +585,20 @@ __device__ __forceinline__ void scalar_transport_cell(const ScalarXport<T>& P, i
         const float dtr = step_dt(P), s = 0.5f * dtr;
         const F3 mid = {p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z};
         const F3 midc = MASK ? clip_from<P2>(d, P.solid, P.halo, cv, p, mid) : mid;
-        const F3 vm = velocity_s<MASK, P2>(d, smp, midc);
+        const F3 vm = velocity_s<EXACT<T, MASK>, P2>(d, smp, midc);
         F3 arr = {p.x - dtr * vm.x, p.y - dtr * vm.y, p.z - dtr * vm.z};
         dep = MASK ? clip_from<P2>(d, P.solid, P.halo, cv, p, arr) : arr;
         if (!same_bits(midc, mid)) {
-            const F3 vm2 = velocity_s<MASK, P2>(d, smp, mid);
+            const F3 vm2 = velocity_s<EXACT<T, MASK>, P2>(d, smp, mid);
             arr = {p.x - dtr * vm2.x, p.y - dtr * vm2.y, p.z - dtr * vm2.z};
         }
         const F3 fdep = {__ldg(P.fdep + i), __ldg(P.fdep + i + P.n), __ldg(P.fdep + i + 2 * P.n)};
         P.ok[i] = scalar_correction_ok<MASK, P2>(d, P.solid, P.halo, cv, p, fdep, mid, arr) ? 1 : 0;
     } else {
-        dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, step_dt(P), cv);
+        dep = backtrace_s<MASK, EXACT<T, MASK>, P2>(d, smp, P.solid, P.halo, p, v0, step_dt(P), cv);
     }
-    float qx = cells<MASK, P2>(d, dep.x, 0) - 0.5f, qy = cells<MASK, P2>(d, dep.y, 1) - 0.5f,
-          qz = cells<MASK, P2>(d, dep.z, 2) - 0.5f;
+    float qx = cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - 0.5f, qy = cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - 0.5f,
+          qz = cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - 0.5f;
     const auto S = smp.template closed<MASK>(P.solid, qx, qy, qz, clear && near_start(d, p, dep));
     for (int c = 0; c < P.count; ++c) Store<T>::st(P.out[c], i, smp.template apply<MASK>(3 + c, S));
     if (P.dep) {
@@ -685,12 +685,12 @@ __device__ __forceinline__ void advect_scalars_cell(const ScalarFinal<T>& P, int
     // the reverse pass decided the correction (scalar_transport_cell with ok)
     const bool decided = reuse && P.ok != nullptr;
     F3 v0 = {0.f, 0.f, 0.f};
-    if (!decided) v0 = start_velocity_cell<MASK, P2>(d, smp, p, x, y, z);
+    if (!decided) v0 = start_velocity_cell<EXACT<T, MASK>, P2>(d, smp, p, x, y, z);
     F3 dep;
     if (reuse) dep = {__ldg(P.dep + i), __ldg(P.dep + i + P.n), __ldg(P.dep + i + 2 * P.n)};
-    else dep = backtrace_s<MASK, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
-    float qx = cells<MASK, P2>(d, dep.x, 0) - 0.5f, qy = cells<MASK, P2>(d, dep.y, 1) - 0.5f,
-          qz = cells<MASK, P2>(d, dep.z, 2) - 0.5f;
+    else dep = backtrace_s<MASK, EXACT<T, MASK>, P2>(d, smp, P.solid, P.halo, p, v0, dt, cv);
+    float qx = cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - 0.5f, qy = cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - 0.5f,
+          qz = cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - 0.5f;
     bool ok = false;
     if (decided) {
         ok = __ldg(P.ok + i) != 0;
@@ -698,7 +698,7 @@ __device__ __forceinline__ void advect_scalars_cell(const ScalarFinal<T>& P, int
         // correct_scalar.glsl:1-21
         float s = 0.5f * dt;
         F3 mid2 = {p.x + s * v0.x, p.y + s * v0.y, p.z + s * v0.z};
-        F3 vm2 = velocity_s<MASK, P2>(d, smp, mid2);
+        F3 vm2 = velocity_s<EXACT<T, MASK>, P2>(d, smp, mid2);
         F3 arr = {p.x + dt * vm2.x, p.y + dt * vm2.y, p.z + dt * vm2.z};
         ok = scalar_correction_ok<MASK, P2>(d, P.solid, P.halo, cv, p, dep, mid2, arr);
     }

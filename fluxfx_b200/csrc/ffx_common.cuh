@@ -206,14 +206,15 @@ __device__ __forceinline__ float dot3(const F3& a, const F3& b) { return (a.x * 
 
 // ---------------------------------------------------------------- samplers
 // How the transport passes form samples and positions.
-//  EXACT samples (face fields of domains with colliders): the sum of eight
-//    rounded weight products in the shaders' order. What such a pass leaves is
-//    the divergence's and the pressure's input, where neighbours cancel, and in
-//    16-bit storage a changed last bit of a sample is a changed 16-bit value now
-//    and then; and where e, n or h is no power of two the MacCormack correction
-//    applies or not according to the last bits of traced positions (within_1e7),
-//    so those quotients by e, n and h are rounded as the division rounds them.
-//  The others (domains without colliders, scalar fields): nested lerps (14 FMAs
+//  EXACT samples (face fields of domains with colliders, all fields in 16-bit
+//    storage): the sum of eight rounded weight products in the shaders' order.
+//    In 16-bit storage a changed last bit of a sample is a changed 16-bit value
+//    now and then, which the divergence, where neighbours cancel, hands on to the
+//    pressure; and with colliders, where e, n or h is no power of two, the
+//    MacCormack correction applies or not according to the last bits of traced
+//    positions (within_1e7). So quotients by e, n and h are rounded there as the
+//    division rounds them.
+//  The others (FP32 domains without colliders, FP32 scalars): nested lerps (14 FMAs
 //    for 28 multiplications and additions), grid coordinates as p (n/e) (one
 //    rounded constant and one product, the two roundings of p n / e, at a tenth
 //    of its instructions), and start points at cell and face centres at their

@@ -119,7 +119,8 @@ __device__ __forceinline__ int floor_int(float v) {
 // stencil (clamped corners, fractions and, with colliders, which corners are
 // fluid and the sum of their weights) is formed once, then applied to each
 // field. Where every corner is fluid (the weights sum to 1) the value is the
-// interpolation; beside a collider, the mean of the fluid corners by weight.
+// interpolation; beside a collider, and in 16-bit storage with colliders, the
+// mean of the fluid corners by weight.
 struct ClosedStencil {
     int rows[4];          // cidx(0, y, z) of (y0, z0), (y1, z0), (y0, z1), (y1, z1)
     int x0, x1;
@@ -130,7 +131,7 @@ struct ClosedStencil {
 
 // fluid: every corner is known to be fluid (a departure point near a clear
 // cell's centre: its corners lie within one cell of it), so the mask is not read.
-template <bool MASK>
+template <bool MASK, bool EXACT>
 __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint8_t* solid, float qx, float qy,
                                                         float qz, bool fluid = false) {
     ClosedStencil S;
@@ -149,13 +150,13 @@ __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint
     S.rows[3] = cidx(d, 0, y1, z1);
     S.fluid = 255u;
     S.total = 1.f;
-    if (MASK && !fluid) {
+    if (MASK && (EXACT || !fluid)) {
         S.fluid = 0u;
         S.total = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int c = S.rows[k >> 1] + ((k & 1) ? S.x1 : S.x0);
-            if (__ldg(solid + c)) continue;
+            if (!fluid && __ldg(solid + c)) continue;
             const float wz = (k & 4) ? S.fz : 1.f - S.fz, wy = (k & 2) ? S.fy : 1.f - S.fy,
                         wx = (k & 1) ? S.fx : 1.f - S.fx;
             S.fluid |= 1u << k;
@@ -165,9 +166,20 @@ __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint
     return S;
 }
 
+// The interpolation between fluid corners; EXACT: products and sums rounded one by one.
+template <bool EXACT>
+__device__ __forceinline__ float closed_value(const float (&c)[8], const ClosedStencil& S) {
+    if (!EXACT) return trilinear<false>(c, S.fx, S.fy, S.fz);
+    const float fx = S.fx, fy = S.fy, fz = S.fz, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
+    const float a0 = c[0] * gx + c[1] * fx, a1 = c[2] * gx + c[3] * fx;
+    const float b0 = c[4] * gx + c[5] * fx, b1 = c[6] * gx + c[7] * fx;
+    return (a0 * gy + a1 * fy) * gz + (b0 * gy + b1 * fy) * fz;
+}
+
 template <typename T, bool MASK>
 __device__ __forceinline__ float apply_closed(const ClosedStencil& S, const T* __restrict__ f) {
-    if (MASK && S.fluid != 255u) {
+    constexpr bool EXACT = sizeof(T) == 2;
+    if (MASK && (EXACT || S.fluid != 255u)) {
         float value = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -182,7 +194,7 @@ __device__ __forceinline__ float apply_closed(const ClosedStencil& S, const T* _
                         Store<T>::ld(f, S.rows[1] + S.x0), Store<T>::ld(f, S.rows[1] + S.x1),
                         Store<T>::ld(f, S.rows[2] + S.x0), Store<T>::ld(f, S.rows[2] + S.x1),
                         Store<T>::ld(f, S.rows[3] + S.x0), Store<T>::ld(f, S.rows[3] + S.x1)};
-    return trilinear<false>(c, S.fx, S.fy, S.fz);
+    return closed_value<EXACT>(c, S);
 }
 
 // ------------------------------------------------------------------ samplers
@@ -289,7 +301,7 @@ struct GlobalSampler {
     template <bool MASK>
     __device__ __forceinline__ ClosedStencil closed(const uint8_t* solid, float qx, float qy, float qz,
                                                     bool fluid = false) const {
-        return closed_stencil<MASK>(f.d, solid, qx, qy, qz, fluid);
+        return closed_stencil<MASK, sizeof(*f.ptr(0)) == 2>(f.d, solid, qx, qy, qz, fluid);
     }
     template <bool MASK>
     __device__ __forceinline__ float apply(int k, const ClosedStencil& S) const {
@@ -354,7 +366,7 @@ struct TileSampler {
     __device__ __forceinline__ Stencil closed(const uint8_t* solid, float qx, float qy, float qz,
                                               bool fluid = false) const {
         Stencil t;
-        t.S = closed_stencil<MASK>(G.f.d, solid, qx, qy, qz, fluid);
+        t.S = closed_stencil<MASK, sizeof(*G.f.ptr(0)) == 2>(G.f.d, solid, qx, qy, qz, fluid);
         const int ix = floor_int(qx), iy = floor_int(qy), iz = floor_int(qz);
         if (tile::inside(w, ix, iy, iz)) {
             const int off = (iy - w.wy) * tile::kPitch + (ix - w.wx);
@@ -377,7 +389,8 @@ struct TileSampler {
             const float* r = (j & 4) ? c1 : c0;
             return r[((j & 2) ? tile::kPitch : 0) + (j & 1)];
         };
-        if (MASK && S.fluid != 255u) {
+        constexpr bool EXACT = sizeof(*G.f.ptr(0)) == 2;
+        if (MASK && (EXACT || S.fluid != 255u)) {
             float value = 0.f;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -389,43 +402,47 @@ struct TileSampler {
             return S.total > 1e-8f ? value / S.total : 0.f;
         }
         const float c[8] = {corner(0), corner(1), corner(2), corner(3), corner(4), corner(5), corner(6), corner(7)};
-        return trilinear<false>(c, S.fx, S.fy, S.fz);
+        return closed_value<EXACT>(c, S);
     }
 };
 
+// Whether the face samples and positions of a domain keep the shaders' operations.
+template <typename T, bool MASK>
+constexpr bool EXACT = MASK || sizeof(T) == 2;
+
 // Grid coordinate of a traced position along axis i.
-template <bool MASK, bool P2>
+template <bool EXACT, bool P2>
 __device__ __forceinline__ float cells(const Dev& d, float x, int i) {
-    return !MASK && !P2 ? x * d.rc[i] : dv_h<P2>(d, x, i);
+    return !EXACT && !P2 ? x * d.rc[i] : dv_h<P2>(d, x, i);
 }
 
 // Staggered velocity at a physical point through a sampler (velocity_at).
-template <bool MASK, bool P2, class S>
+template <bool EXACT, bool P2, class S>
 __device__ __forceinline__ F3 velocity_s(const Dev& d, const S& smp, F3 p) {
     float q[3];
     const float pp[3] = {p.x, p.y, p.z};
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        if (MASK && !P2)      // beyond 2^96 (or not a number) the sample's clamp decides
+        if (EXACT && !P2)      // beyond 2^96 (or not a number) the sample's clamp decides
             q[i] = div_near(fminf(fmaxf(pp[i] * d.nf[i], -0x1p96f), 0x1p96f), d.e[i], d.re[i]);
         else
             q[i] = pp[i] * d.rc[i];
     }
     F3 r;
-    r.x = smp.template sample<MASK>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
-    r.y = smp.template sample<MASK>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
-    r.z = smp.template sample<MASK>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
+    r.x = smp.template sample<EXACT>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
+    r.y = smp.template sample<EXACT>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
+    r.z = smp.template sample<EXACT>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
     return r;
 }
 
 // Velocity at the face centre p = (X2, Y2, Z2) / 2 cells.
-template <bool MASK, bool P2, class S>
+template <bool EXACT, bool P2, class S>
 __device__ __forceinline__ F3 start_velocity_s(const Dev& d, const S& smp, F3 p, int X2, int Y2, int Z2) {
-    if constexpr (!MASK || P2) {
+    if constexpr (!EXACT || P2) {
         F3 r;
-        r.x = smp.template half<MASK>(0, X2, Y2 - 1, Z2 - 1);
-        r.y = smp.template half<MASK>(1, X2 - 1, Y2, Z2 - 1);
-        r.z = smp.template half<MASK>(2, X2 - 1, Y2 - 1, Z2);
+        r.x = smp.template half<EXACT>(0, X2, Y2 - 1, Z2 - 1);
+        r.y = smp.template half<EXACT>(1, X2 - 1, Y2, Z2 - 1);
+        r.z = smp.template half<EXACT>(2, X2 - 1, Y2 - 1, Z2);
         return r;
     } else {
         return velocity_s<true, false>(d, smp, p);
@@ -433,11 +450,11 @@ __device__ __forceinline__ F3 start_velocity_s(const Dev& d, const S& smp, F3 p,
 }
 
 // Velocity at the centre p of cell (x, y, z): the two faces along each axis.
-template <bool MASK, bool P2, class S>
+template <bool EXACT, bool P2, class S>
 __device__ __forceinline__ F3 start_velocity_cell(const Dev& d, const S& smp, F3 p, int x, int y, int z) {
-    if constexpr (!MASK || P2)
-        return F3{smp.template node<MASK, 1, 0, 0>(0, x, y, z), smp.template node<MASK, 0, 1, 0>(1, x, y, z),
-                  smp.template node<MASK, 0, 0, 1>(2, x, y, z)};
+    if constexpr (!EXACT || P2)
+        return F3{smp.template node<EXACT, 1, 0, 0>(0, x, y, z), smp.template node<EXACT, 0, 1, 0>(1, x, y, z),
+                  smp.template node<EXACT, 0, 0, 1>(2, x, y, z)};
     else
         return velocity_s<true, false>(d, smp, p);
 }
@@ -448,34 +465,34 @@ __device__ __forceinline__ F3 start_velocity_cell(const Dev& d, const S& smp, F3
 // and the parities of every component's node are fixed by the axis: the U face
 // (2x, 2y+1, 2z+1) reads u at (x, y, z), v at (x-1..x, y..y+1, z) and w at
 // (x-1..x, y, z..z+1), and likewise for V and W faces.
-template <bool MASK, bool P2, class S>
+template <bool EXACT, bool P2, class S>
 __device__ __forceinline__ F3 start_velocity_face(const Dev& d, const S& smp, F3 p, int axis, int x, int y, int z) {
-    if constexpr (!MASK || P2) {
+    if constexpr (!EXACT || P2) {
         const int c = axis == 0 ? x : (axis == 1 ? y : z);
         const int n = axis == 0 ? d.nx : (axis == 1 ? d.ny : d.nz);
         if (c >= 1 && c <= n - 1) {
             if (axis == 0)
-                return F3{smp.template node<MASK, 0, 0, 0>(0, x, y, z), smp.template node<MASK, 1, 1, 0>(1, x - 1, y, z),
-                          smp.template node<MASK, 1, 0, 1>(2, x - 1, y, z)};
+                return F3{smp.template node<EXACT, 0, 0, 0>(0, x, y, z), smp.template node<EXACT, 1, 1, 0>(1, x - 1, y, z),
+                          smp.template node<EXACT, 1, 0, 1>(2, x - 1, y, z)};
             if (axis == 1)
-                return F3{smp.template node<MASK, 1, 1, 0>(0, x, y - 1, z), smp.template node<MASK, 0, 0, 0>(1, x, y, z),
-                          smp.template node<MASK, 0, 1, 1>(2, x, y - 1, z)};
-            return F3{smp.template node<MASK, 1, 0, 1>(0, x, y, z - 1), smp.template node<MASK, 0, 1, 1>(1, x, y, z - 1),
-                      smp.template node<MASK, 0, 0, 0>(2, x, y, z)};
+                return F3{smp.template node<EXACT, 1, 1, 0>(0, x, y - 1, z), smp.template node<EXACT, 0, 0, 0>(1, x, y, z),
+                          smp.template node<EXACT, 0, 1, 1>(2, x, y - 1, z)};
+            return F3{smp.template node<EXACT, 1, 0, 1>(0, x, y, z - 1), smp.template node<EXACT, 0, 1, 1>(1, x, y, z - 1),
+                      smp.template node<EXACT, 0, 0, 0>(2, x, y, z)};
         }
     }
-    return start_velocity_s<MASK, P2>(d, smp, p, 2 * x + (axis != 0), 2 * y + (axis != 1), 2 * z + (axis != 2));
+    return start_velocity_s<EXACT, P2>(d, smp, p, 2 * x + (axis != 0), 2 * y + (axis != 1), 2 * z + (axis != 2));
 }
 
 // Midpoint backtrace through a sampler (the `backtrace` of the transport
 // passes); `cv`: the clearance of the start point's own cell (home_clearance).
-template <bool MASK, bool P2, class S>
+template <bool MASK, bool EXACT, bool P2, class S>
 __device__ __forceinline__ F3 backtrace_s(const Dev& d, const S& smp, const uint8_t* solid, const uint8_t* halo, F3 p,
                                           F3 v0, float dt, int cv = 0) {
     const float s = 0.5f * dt;
     F3 mid = {p.x - s * v0.x, p.y - s * v0.y, p.z - s * v0.z};
     if (MASK) mid = clip_from<P2>(d, solid, halo, cv, p, mid);
-    const F3 vm = velocity_s<MASK, P2>(d, smp, mid);
+    const F3 vm = velocity_s<EXACT, P2>(d, smp, mid);
     F3 dep = {p.x - dt * vm.x, p.y - dt * vm.y, p.z - dt * vm.z};
     if (MASK) dep = clip_from<P2>(d, solid, halo, cv, p, dep);
     return dep;
