@@ -4,7 +4,8 @@ Drop-in for FluxFX ``fluxfx/backend/multigrid.py:6-106``: weighted Jacobi
 (omega = 2/3), rediscretised Neumann Laplacian per level, 2x2x2 averaging,
 clamped trilinear prolongation, coarse levels solved with dt = 1, and the 4^3
 closed-form pseudoinverse on the coarsest level. All cycles of a fixed budget
-are one native call (``relax.Relaxation``).
+are one native call (``relax.Relaxation``); with 16-bit storage a launch per
+pass, residual and restriction as one.
 Extensions (``PressureSettings``): sweep counts, a level cap (the coarsest
 level up to 512 cells then uses the same closed-form inverse in FP64), and
 cycling to a relative max-norm tolerance.
@@ -52,9 +53,9 @@ class MultigridPressureProjector(PressureProjector):
         for i, shape in enumerate(shapes):
             self.levels.append({
                 'shape': shape, 'inv': tuple(n / e for n, e in zip(shape, grid.extent)),
-                'p': self.pressure if i == 0 else None,
-                'q': self.spare if i == 0 else None,
-                'rhs': self.before if i == 0 else None,
+                'p': self.pressure if i == 0 else dev.texture(shape) if self._separate_passes else None,
+                'q': self.spare if i == 0 else dev.texture(shape) if self._separate_passes else None,
+                'rhs': self.before if i == 0 else dev.texture(shape) if self._separate_passes else None,
                 'residual': None})
         coarsest = shapes[-1]
         if len(shapes) > 1 and s.coarse_solver == 'DIRECT' and (
@@ -68,7 +69,8 @@ class MultigridPressureProjector(PressureProjector):
         self.post_sweeps = s.mg_post_sweeps or 3
         # the levels below the first live inside the native cycles
         self._relaxation = Relaxation(dev, shapes, grid.extent, 2.0 / 3.0, pre=self.pre_sweeps, post=self.post_sweeps,
-                                      last=80, basis=self.coarse_basis) if len(shapes) > 1 else None
+                                      last=80, basis=self.coarse_basis) if (
+            len(shapes) > 1 and not self._separate_passes) else None
         self._cycle_sweeps = (len(shapes) - 1) * (self.pre_sweeps + self.post_sweeps) + (
             0 if self.coarse_basis is not None else 80)
         self.last_cycles = 0
@@ -77,13 +79,18 @@ class MultigridPressureProjector(PressureProjector):
 
     @property
     def allocated_bytes(self):
-        extra = self._relaxation.allocated_bytes if self._relaxation is not None else 0
+        extra = self._relaxation.allocated_bytes if self._relaxation is not None else 4 * sum(
+            3 * prod(v['shape']) for v in self.levels[1:])
         return super().allocated_bytes + extra + sum(
             8 * t.numel() for t in (self.coarse_matrix, self.coarse_basis) if t is not None)
 
     def reset(self):
         super().reset()
         self.last_cycles = 0
+        for level in self.levels[1:]:
+            for name in ('p', 'q', 'rhs'):
+                if level[name] is not None:
+                    level[name].zero_()
 
     def _n3(self, level):
         return N.n3(*level['shape'])
@@ -91,14 +98,51 @@ class MultigridPressureProjector(PressureProjector):
     def _inv3(self, level):
         return N.f3(*level['inv'])
 
+    def smooth(self, level, dt, count):
+        s = self.device.s
+        for _ in range(count):
+            self.device.call('ffx_jacobi', self._n3(level), self._inv3(level), None, ptr(level['p']),
+                             ptr(level['rhs']), dt, 2.0 / 3.0, ptr(level['q']), s)
+            level['p'], level['q'] = level['q'], level['p']
+
+    def cycle(self, index, dt):
+        """One V-cycle, a launch per pass."""
+        level = self.levels[index]
+        s = self.device.s
+        if index == len(self.levels) - 1:
+            if self.coarse_matrix is not None:
+                self.device.call('ffx_direct_solve', prod(level['shape']), ptr(self.coarse_matrix),
+                                 ptr(level['rhs']), dt, ptr(level['p']), s)
+            else:
+                self.smooth(level, dt, 80)
+            return
+        self.smooth(level, dt, self.pre_sweeps)
+        coarse = self.levels[index + 1]
+        self.device.call('ffx_mg_residual_restrict', self._n3(level), self._inv3(level), ptr(level['p']),
+                         ptr(level['rhs']), dt, ptr(coarse['rhs']), s)
+        coarse['p'].zero_()
+        self.cycle(index + 1, 1.0)
+        self.device.call('ffx_mg_prolong', self._n3(level), ptr(level['p']), ptr(coarse['p']), ptr(level['q']), s)
+        level['p'], level['q'] = level['q'], level['p']
+        self.smooth(level, dt, self.post_sweeps)
+
     def _cycles(self, count, dt, from_zero=False):
         """``count`` V-cycles on level 0's iterate (not read when ``from_zero``)."""
         level = self.levels[0]
-        level['p'], level['q'] = self._relaxation.run(level['p'], level['q'], level['rhs'], count, dt, from_zero)
+        if self._separate_passes:
+            if from_zero:
+                level['p'].zero_()
+            for _ in range(count):
+                self.cycle(0, dt)
+        else:
+            self._relax(level, count, dt, from_zero)
         self.last_cycles += count
         self.last_iterations += count * self._cycle_sweeps
         if self.coarse_basis is not None:
             self.last_coarse_solves += count
+
+    def _relax(self, level, count, dt, from_zero):
+        level['p'], level['q'] = self._relaxation.run(level['p'], level['q'], level['rhs'], count, dt, from_zero)
 
     def _residual_max(self, dt):
         level = self.levels[0]

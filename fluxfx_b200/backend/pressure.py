@@ -29,6 +29,10 @@ class PressureProjector:
         self._field_dtype = torch.bfloat16 if self.settings.storage == 'BF16' else torch.float32
         self._storage = N.FFX_F32 if self._field_dtype == torch.float32 else N.FFX_BF16
         self._mask = getattr(self.device, 'mask', None)
+        # 16-bit storage keeps a launch per pass: the whole-solve kernels round their
+        # sums in another order, and a pressure whose last bit differs flips stored
+        # 16-bit velocities, which the next step's divergence shows (1e-4 of its pressure)
+        self._separate_passes = self._storage == N.FFX_BF16
         self._jacobi = None       # the Jacobi solve's plan (made on first use)
         self._classes = None      # open-neighbour codes of the mask (ffx_relax_classes)
         self._solids = solids_struct(self.device)
@@ -236,6 +240,15 @@ class PressureProjector:
         scaled = ceil(self.settings.pressure_iterations * max(1.0, (max(self.grid.shape) / 64) ** 2))
         multiplier = self.settings.pressure_cold_multiplier if previous_dt != dt else 1
         self.last_iterations = min(4096, scaled * multiplier)
+        if self._separate_passes:
+            if self._starts_from_zero(dt, previous_dt):
+                self.pressure.zero_()
+            omega = self.settings.pressure_relaxation
+            for _ in range(self.last_iterations):
+                self.device.call('ffx_jacobi', self._n3, self._inv3, self._mask_ptr(), ptr(self.pressure),
+                                 ptr(self.before), dt, omega, ptr(self.spare), self.device.s)
+                self.pressure, self.spare = self.spare, self.pressure
+            return
         if self._jacobi is None:
             if self._mask is not None:
                 nx, ny, nz = self.grid.shape
