@@ -37,6 +37,7 @@ enum Mode { kSweeps = 0, kDown = 1, kUp = 2 };
 
 using resident::byte_of;
 using resident::fill_table;
+using resident::weighted;
 using resident::weights_of;
 using resident::zero4;
 
@@ -145,7 +146,7 @@ __device__ __forceinline__ void sweep(const Box& b, const Lane& l, const Weights
             lo = c;
             c = hi;
         }
-        Q[i] = out;
+        Q[i] = weighted(k, out);
     }
 }
 

@@ -92,6 +92,13 @@ __device__ __forceinline__ void weights_of(unsigned codes, const float2* kd, flo
     d = make_float4(a.y, b.y, c.y, e.y);
 }
 
+// A sweep's result: 0 in the cells without a weight (colliders, isolated cells,
+// padding), whatever stands beside them. Selected, not multiplied: 0 times an
+// infinity would carry it through a wall.
+__device__ __forceinline__ float4 weighted(float4 k, float4 o) {
+    return make_float4(k.x > 0.f ? o.x : 0.f, k.y > 0.f ? o.y : 0.f, k.z > 0.f ? o.z : 0.f, k.w > 0.f ? o.w : 0.f);
+}
+
 // n / d for 0 <= n < 2^16 and 1 <= d < 2^12, with inv = 1 / d: (n + 1/2) / d is
 // at least 1 / (2 d) from an integer, far more than the rounding.
 __device__ __forceinline__ int quotient(int n, float inv) { return __float2int_rd(((float)n + 0.5f) * inv); }
@@ -288,7 +295,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             const int gz = v.z0 + z0 + j;
             if (gz == 0 || gz == v.n[2] - 1) weights_of(edge, kd, k, d);
         }
-        if (blank) return make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w);
+        if (blank) return weighted(k, make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w));
         const float4 ym = P[i - v.x4], yp = P[i + v.x4];
         const float* row = reinterpret_cast<const float*>(P) + 4 * i;
         const float xl = left ? row[-1] : 0.f, xr = right ? row[4] : 0.f;
@@ -301,7 +308,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
                         fmaf(k.z, fmaf(-d.z, c.z, o.z), c.z), fmaf(k.w, fmaf(-d.w, c.w, o.w), c.w));
         lo = c;
         c = hi;
-        return o;
+        return weighted(k, o);
     };
     for (int s = 0; s < count; ++s) {
         const bool blank = zero && s == 0;
