@@ -222,19 +222,25 @@ __device__ __forceinline__ float dot3(const F3& a, const F3& b) { return (a.x * 
 // The passes are bound by instruction issue (75-87 % of the slots; DRAM under
 // 17 %), so instructions are what a sample costs. Measured, all transport passes
 // of a step, clamped corners one by one and weighted sums everywhere -> this:
-// 128 x 96 x 112 FP32 without colliders 455 -> 318 us; with colliders, 256^3 BF16
+// 128 x 96 x 112 FP32 without colliders 455 -> 328 us; with colliders, 256^3 BF16
 // 4.8 -> 4.1 ms and 96 x 80 x 112 FP32 470 -> 446 us.
 
-// (1 - t) a + t b: exactly a at t = 0 and b at t = 1.
+// (1 - t) a + t b: exactly a at t = 0 and b at t = 1, for finite a and b.
 __device__ __forceinline__ float lerp(float a, float b, float t) { return fmaf(t, b, fmaf(-t, a, a)); }
+// The same with g = 1 - t: an infinity that has a weight stays one (a - t a is a NaN).
+__device__ __forceinline__ float lerp(float a, float b, float g, float t) { return fmaf(t, b, g * a); }
 
 // Interpolation between eight corner values, corner k at bit 0 = x, bit 1 = y, bit 2 = z.
-template <bool EXACT>
+// FINITE: in the short form where it is not EXACT, for finite corners.
+template <bool EXACT, bool FINITE>
 __device__ __forceinline__ float trilinear(const float (&c)[8], float fx, float fy, float fz) {
-    if (!EXACT)
+    if (!EXACT && FINITE)
         return lerp(lerp(lerp(c[0], c[1], fx), lerp(c[2], c[3], fx), fy),
                     lerp(lerp(c[4], c[5], fx), lerp(c[6], c[7], fx), fy), fz);
     const float gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
+    if (!EXACT)
+        return lerp(lerp(lerp(c[0], c[1], gx, fx), lerp(c[2], c[3], gx, fx), gy, fy),
+                    lerp(lerp(c[4], c[5], gx, fx), lerp(c[6], c[7], gx, fx), gy, fy), gz, fz);
     float v = 0.f;
     v = v + gx * gy * gz * c[0];
     v = v + fx * gy * gz * c[1];
@@ -275,7 +281,7 @@ __device__ __forceinline__ void cube_range(const float (&c)[8], float& lo, float
 // Lower corner and fraction of coordinate q clamped to [0, s - 1] along an axis
 // of s samples, the corner at most s - 2 (the fraction at the upper edge is 1,
 // which weights the same samples with the same numbers in the same order as a
-// clamped upper corner does). 2^23 + q rounded toward zero is 2^23 + floor(q), so
+// clamped upper corner does, and the sample before them with 0). 2^23 + q rounded toward zero is 2^23 + floor(q), so
 // neither floor nor conversion runs in the quarter-rate unit; `bits` is the
 // corner plus kCornerBias.
 constexpr unsigned kCornerBias = 0x4b000000u;
@@ -293,14 +299,45 @@ __device__ __forceinline__ int corner_index(Corner x, Corner y, Corner z, int sx
     return (int)(x.bits + ux * (y.bits + uy * z.bits) - kCornerBias * (1u + ux * (1u + uy)));
 }
 
-// Clamped trilinear sample of a face grid of size (sx, sy, sz) (mac_sample.glsl:2-19).
+// Clamped trilinear sample of a face grid of size (sx, sy, sz) (mac_sample.glsl:2-19),
+// both corners clamped to the field: at its upper edge the last sample counts alone.
 template <bool EXACT, typename T>
-__device__ __forceinline__ float sample_face(const T* __restrict__ f, int sx, int sy, int sz,
+__device__ __noinline__ float sample_clamped(const T* f, int sx, int sy, int sz, float qx, float qy, float qz) {
+    qx = fminf(fmaxf(qx, 0.f), (float)(sx - 1));
+    qy = fminf(fmaxf(qy, 0.f), (float)(sy - 1));
+    qz = fminf(fmaxf(qz, 0.f), (float)(sz - 1));
+    const float bx = floorf(qx), by = floorf(qy), bz = floorf(qz);
+    const int x0 = (int)bx, y0 = (int)by, z0 = (int)bz;
+    const int x1 = min(x0 + 1, sx - 1), y1 = min(y0 + 1, sy - 1), z1 = min(z0 + 1, sz - 1);
+    float c[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        c[k] = Store<T>::ld(f, (k & 1 ? x1 : x0) + sx * ((k & 2 ? y1 : y0) + sy * (k & 4 ? z1 : z0)));
+    return trilinear<EXACT, false>(c, qx - bx, qy - by, qz - bz);
+}
+
+// The same value in fewer instructions where all samples around the point are finite.
+// Where one is not, the result may be a NaN too many: the sample before the last has
+// the weight 0 at the upper edge, and the short lerps spoil an infinity. So a result
+// that is not finite is formed again, out of line. (Measured, us per step, without the
+// test -> with it: 128 x 96 x 112 FP32 without colliders 535 -> 545, with colliders
+// 96 x 80 x 112 FP32 682 -> 682, 256^3 BF16 7366 -> 7469. Testing the coordinates for the edge instead, in the
+// longer lerps, took 550 and 706: a branch before a sum keeps the loads of the next
+// sample behind it.)
+template <bool EXACT, typename T>
+__device__ __forceinline__ float sample_near(const T* __restrict__ f, int sx, int sy, int sz,
                                              float qx, float qy, float qz) {
     const Corner x = lower_corner(qx, sx), y = lower_corner(qy, sy), z = lower_corner(qz, sz);
     float c[8];
     load_cube(f, sx, sy, sz, corner_index(x, y, z, sx, sy), c);
-    return trilinear<EXACT>(c, x.f, y.f, z.f);
+    return trilinear<EXACT, true>(c, x.f, y.f, z.f);
+}
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 0x1.fffffep127f; }
+template <bool EXACT, typename T>
+__device__ __forceinline__ float sample_face(const T* __restrict__ f, int sx, int sy, int sz,
+                                             float qx, float qy, float qz) {
+    const float v = sample_near<EXACT>(f, sx, sy, sz, qx, qy, qz);
+    return finite(v) ? v : sample_clamped<EXACT>(f, sx, sy, sz, qx, qy, qz);
 }
 
 template <typename T>

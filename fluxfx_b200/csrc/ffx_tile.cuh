@@ -90,7 +90,8 @@ __device__ __forceinline__ float sample(const Window& w, int k, const T* __restr
     const Corners c = corners(w, k, ix, iy, iz);
     const float v[8] = {c.c0[0], c.c0[1], c.c0[kPitch], c.c0[kPitch + 1], c.c1[0], c.c1[1], c.c1[kPitch],
                         c.c1[kPitch + 1]};
-    return trilinear<EXACT>(v, qx - bx, qy - by, qz - bz);
+    const float r = trilinear<EXACT, true>(v, qx - bx, qy - by, qz - bz);
+    return finite(r) ? r : sample_clamped<EXACT>(g, sx, sy, sz, qx, qy, qz);
 }
 
 // sample_face_half (a node sample: doubled coordinates) of field k.
@@ -169,7 +170,7 @@ __device__ __forceinline__ ClosedStencil closed_stencil(const Dev& d, const uint
 // The interpolation between fluid corners; EXACT: products and sums rounded one by one.
 template <bool EXACT>
 __device__ __forceinline__ float closed_value(const float (&c)[8], const ClosedStencil& S) {
-    if (!EXACT) return trilinear<false>(c, S.fx, S.fy, S.fz);
+    if (!EXACT) return trilinear<false, false>(c, S.fx, S.fy, S.fz);
     const float fx = S.fx, fy = S.fy, fz = S.fz, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
     const float a0 = c[0] * gx + c[1] * fx, a1 = c[2] * gx + c[3] * fx;
     const float b0 = c[4] * gx + c[5] * fx, b1 = c[6] * gx + c[7] * fx;
@@ -247,6 +248,19 @@ struct GlobalSampler {
         int sx, sy, sz;
         f.dims(k, sx, sy, sz);
         return sample_face<EXACT>(f.ptr(k), sx, sy, sz, qx, qy, qz);
+    }
+    // its two parts: `near`, and where that is not finite `clamped`
+    template <bool EXACT>
+    __device__ __forceinline__ float near(int k, float qx, float qy, float qz) const {
+        int sx, sy, sz;
+        f.dims(k, sx, sy, sz);
+        return sample_near<EXACT>(f.ptr(k), sx, sy, sz, qx, qy, qz);
+    }
+    template <bool EXACT>
+    __device__ __forceinline__ float clamped(int k, float qx, float qy, float qz) const {
+        int sx, sy, sz;
+        f.dims(k, sx, sy, sz);
+        return sample_clamped<EXACT>(f.ptr(k), sx, sy, sz, qx, qy, qz);
     }
     template <bool EXACT>
     __device__ __forceinline__ float half(int k, int qx2, int qy2, int qz2) const {
@@ -326,6 +340,14 @@ struct TileSampler {
         int sx, sy, sz;
         G.f.dims(k, sx, sy, sz);
         return tile::sample<EXACT>(w, k, G.f.ptr(k), sx, sy, sz, qx, qy, qz);
+    }
+    template <bool EXACT>
+    __device__ __forceinline__ float near(int k, float qx, float qy, float qz) const {
+        return sample<EXACT>(k, qx, qy, qz);
+    }
+    template <bool EXACT>
+    __device__ __forceinline__ float clamped(int k, float qx, float qy, float qz) const {
+        return sample<EXACT>(k, qx, qy, qz);
     }
     template <bool EXACT>
     __device__ __forceinline__ float half(int k, int qx2, int qy2, int qz2) const {
@@ -429,9 +451,15 @@ __device__ __forceinline__ F3 velocity_s(const Dev& d, const S& smp, F3 p) {
             q[i] = pp[i] * d.rc[i];
     }
     F3 r;
-    r.x = smp.template sample<EXACT>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
-    r.y = smp.template sample<EXACT>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
-    r.z = smp.template sample<EXACT>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
+    r.x = smp.template near<EXACT>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
+    r.y = smp.template near<EXACT>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
+    r.z = smp.template near<EXACT>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
+    // one test for the three: their sum is not finite where one of them is not
+    if (!finite(fabsf(r.x) + fabsf(r.y) + fabsf(r.z))) {
+        r.x = smp.template clamped<EXACT>(0, q[0], q[1] - 0.5f, q[2] - 0.5f);
+        r.y = smp.template clamped<EXACT>(1, q[0] - 0.5f, q[1], q[2] - 0.5f);
+        r.z = smp.template clamped<EXACT>(2, q[0] - 0.5f, q[1] - 0.5f, q[2]);
+    }
     return r;
 }
 
