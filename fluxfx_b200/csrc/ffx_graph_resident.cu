@@ -177,6 +177,7 @@ int fill(const Spec& S, int dist, const Candidate& c, int first_block, u64* ws, 
         L.base.p = L.base.q = off;
         off += rim;
         if (k < dist) {
+            D.exchanges += k == S.count - 1 ? S.last : (k == 0 ? S.pre0 + S.post0 : S.pre + S.post);
             L.base.ll = word;
             word += 2 * 4 * slots_of(S.level[k]);
             if (k == 0 && S.whole) {

@@ -68,6 +68,7 @@ struct Domain {
     u64* ws;
     int64_t tail_rhs, tail_p, maxima, control;   // words
     unsigned* epochs;                  // two per block: exchange and tail numbers reached
+    int exchanges;                     // of a cycle's sweeps, all levels in tiles
     unsigned* timeouts;
     int tile_f4, tail_f4;
     double tol;
@@ -89,6 +90,20 @@ struct Call {
     int aligned;         // p and rhs start on 16 bytes
     int batched;         // everything from the domains' own records
 };
+
+// Cycles of a launch at most.
+__device__ __forceinline__ int cycle_limit(const Domain& D, const Call& A) {
+    if (!D.whole) return 1;
+    return A.cycles > 0 ? A.cycles : (A.batched ? D.max_cycles : A.max_cycles);
+}
+// What a launch adds to a block's two numbers: as many exchanges (every sweep's, a
+// maximum per decision, the scale) and decisions as it may take, not those it took.
+// So a wait that gives up, after which blocks may part ways, leaves them with the
+// same numbers for the next launch.
+__device__ __forceinline__ unsigned exchanges_numbered(const Domain& D, int limit) {
+    return 2u + (unsigned)limit * (unsigned)(D.exchanges + 1);
+}
+__device__ __forceinline__ unsigned decisions_numbered(int limit) { return (unsigned)limit + 1u; }
 
 struct GView {
     View v;
@@ -485,7 +500,8 @@ __device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4*
         if (k != last || !D.inverse) divide |= (load_edges(D.tv[k], view(k), smem) ? 1u : 0u) << k;
     const GView top = view(first);
     const int slots = top.v.flat * top.v.tz;
-    unsigned number = D.epochs[2 * block + 1];
+    const unsigned base = D.epochs[2 * block + 1];
+    unsigned number = base;
     __shared__ int go;
     for (int c = 0;; ++c) {
         ++number;
@@ -556,7 +572,7 @@ __device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4*
         }
     }
     __syncthreads();
-    if (tid == 0) D.epochs[2 * block + 1] = number;
+    if (tid == 0) D.epochs[2 * block + 1] = base + decisions_numbered(cycle_limit(D, A));
 }
 
 // LINKS: the domain's level 0 is the mask's grid (a whole solve); else it is a
@@ -568,13 +584,14 @@ __device__ __forceinline__ void run_tile(const Domain& D, const Call& A, float4*
     const int by = tile % D.gy, bz = tile / D.gy;
     unsigned flip = 0;
     auto view = [&](int k) { return make_gview(D, D.lv[k], by, bz, smem, D.ws, flip >> k & 1u); };
-    Exchange ex = {true, D.epochs[2 * tile] + 1u, 0u, dead, D.timeouts};
-    unsigned number = D.epochs[2 * tile + 1], turn = 0;
+    const unsigned ex_base = D.epochs[2 * tile], base = D.epochs[2 * tile + 1];
+    Exchange ex = {true, ex_base + 1u, 0u, dead, D.timeouts};
+    unsigned number = base, turn = 0;
     float* const P_out = A.batched ? D.p : A.p;
     const float* const rhs = A.batched ? D.rhs : A.rhs;
     const bool from_zero = !LINKS || (!A.batched && A.from_zero);
     const bool to_tolerance = LINKS && A.cycles == 0;
-    const int limit = !LINKS ? 1 : (to_tolerance ? (A.batched ? D.max_cycles : A.max_cycles) : A.cycles);
+    const int limit = cycle_limit(D, A);
     const double tol = A.batched ? D.tol : A.tol;
     const bool vec = D.vec && A.aligned;
     float scale = 0.f;
@@ -752,8 +769,8 @@ __device__ __forceinline__ void run_tile(const Domain& D, const Call& A, float4*
     }
     __syncthreads();
     if (tid == 0) {
-        D.epochs[2 * tile] = ex.epoch;
-        D.epochs[2 * tile + 1] = number;
+        D.epochs[2 * tile] = ex_base + exchanges_numbered(D, limit);
+        D.epochs[2 * tile + 1] = base + decisions_numbered(limit);
         if (tile == 0 && to_tolerance) {
             if (A.batched) {
                 D.state->cycles = c;
