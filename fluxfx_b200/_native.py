@@ -68,7 +68,8 @@ GRAPH_PLAN_LEVELS = 10
 class FfxGraphPlan(C.Structure):
     _fields_ = [('count', i32), ('pre0', i32), ('post0', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32),
                 ('omega', f32), ('inverse', vp), ('level', FfxGraphLevel * GRAPH_PLAN_LEVELS), ('blocks', i32),
-                ('tile', i32 * 2), ('tail', i32), ('shared_bytes', i32), ('workspace_bytes', i64), ('workspace', vp)]
+                ('tile', i32 * 2), ('tail', i32), ('shared_bytes', i32), ('workspace_bytes', i64), ('workspace', vp),
+                ('alarm', vp)]
 
 
 TAIL_LEVELS = 8
@@ -103,7 +104,7 @@ class FfxRelaxLevel(C.Structure):
 class FfxRelaxPlan(C.Structure):
     _fields_ = [('count', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32), ('tail', i32), ('tile', i32 * 2),
                 ('omega', f32), ('basis', vp), ('classes', vp), ('workspace_bytes', i64), ('workspace', vp),
-                ('level', FfxRelaxLevel * RELAX_LEVELS)]
+                ('level', FfxRelaxLevel * RELAX_LEVELS), ('alarm', vp)]
 
 
 class FfxBrickStats(C.Structure):
@@ -282,6 +283,7 @@ _PROTOTYPES = {
     'ffx_relax_plan': (C.c_int, [P(FfxRelaxPlan)]),
     'ffx_relax_cycles': (C.c_int, [P(FfxRelaxPlan), i32, f32, i32, P(i32), vp]),
     'ffx_relax_timeouts': (C.c_int, [P(FfxRelaxPlan), P(i32), vp]),
+    'ffx_relax_reset': (C.c_int, [P(FfxRelaxPlan), vp]),
     'ffx_relax_classes': (C.c_int, [n3, vp, vp, vp]),
     'ffx_graph_smooth': (C.c_int, [P(FfxGraphLevel), vp, vp, f32, vp, vp]),
     'ffx_graph_smooth2': (C.c_int, [P(FfxGraphLevel), vp, vp, f32, vp, vp, vp]),
@@ -301,6 +303,7 @@ _PROTOTYPES = {
     'ffx_graph_plan_upload': (C.c_int, [P(FfxGraphPlan), vp]),
     'ffx_graph_solve': (C.c_int, [P(FfxGraphPlan), vp, vp, i32, i32, C.c_double, i32, vp, vp]),
     'ffx_graph_plan_timeouts': (C.c_int, [P(FfxGraphPlan), P(i32), vp]),
+    'ffx_graph_plan_reset': (C.c_int, [P(FfxGraphPlan), vp]),
     'ffx_conv_forward': (C.c_int, [P(FfxConv), vp]),
     'ffx_conv_forward_tc': (C.c_int, [P(FfxConv), vp]),
     'ffx_conv_timeouts': (C.c_int, [P(i32), i32]),

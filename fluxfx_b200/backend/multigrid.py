@@ -144,6 +144,11 @@ class MultigridPressureProjector(PressureProjector):
     def _relax(self, level, count, dt, from_zero):
         level['p'], level['q'] = self._relaxation.run(level['p'], level['q'], level['rhs'], count, dt, from_zero)
 
+    def check_waits(self):
+        super().check_waits()
+        if self._relaxation is not None:
+            self._relaxation.check()
+
     def _residual_max(self, dt):
         level = self.levels[0]
         self.device.call('ffx_mg_residual_max', self._n3(level), self._inv3(level), ptr(level['p']),

@@ -265,10 +265,19 @@ class PressureProjector:
         self.pressure, self.spare = self._jacobi.run(self.pressure, self.spare, self.before, 1, dt,
                                                      self._starts_from_zero(dt, previous_dt))
 
+    def check_waits(self):
+        """Raises FFX_ERR_TIMEOUT when a bounded wait of a solve that the GPU has
+        finished gave up (its pressure is wrong; the next solve is right again).
+        Every solve looks first, and every readback afterwards."""
+        if self._jacobi is not None:
+            self._jacobi.check()
+
     # ------------------------------------------------------------- diagnostics
     def velocity_maxima(self):
         """max |u|, |v|, |w| of the last corrected velocity (one readback)."""
-        return [float(v) for v in self.device.fetch(self._scalars[0:3])]
+        maxima = [float(v) for v in self.device.fetch(self._scalars[0:3])]
+        self.check_waits()
+        return maxima
 
     def divergence_summary(self):
         """FP64 statistics of ``before``/``after`` on the device (one readback)."""
@@ -283,6 +292,7 @@ class PressureProjector:
         self.device.call('ffx_divergence_stats', n, ptr(self.before), ptr(self.after), ptr(out), ptr(ws),
                          ws.numel() * 8, self.device.s)
         b2, a2, mb, ma, sb, sa, count, _ = out.cpu().tolist()
+        self.check_waits()
         rms_b, rms_a = (b2 / count) ** 0.5, (a2 / count) ** 0.5
         ratio = rms_a / rms_b if rms_b > 0 else (0.0 if rms_a == 0 else None)
         out = {"rms_before": rms_b, "rms_after": rms_a, "ratio": ratio, "max_before": mb, "max_after": ma,

@@ -20,6 +20,7 @@ import torch
 from .. import _native as N
 from .collision import SolidPressureProjector
 from .device import KernelHandle, ptr
+from .relax import Alarm
 
 DIRECT_LIMIT = 256
 TAIL_CELLS = 512   # coarse levels at most this size run in one single-block launch
@@ -114,6 +115,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         # pre-sweep (ffx_graph_residual_max_smooth; same results)
         self.speculate = True
         self._pending_refresh = None
+        self._alarm = None       # of the resident plans (made with the first)
         self._loops = {}
         # [cycles of the last solve, cycles of all device-loop solves, decisions]
         self._counters = torch.zeros(3, dtype=torch.int32, device=dev.device)
@@ -130,6 +132,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         if getattr(self, '_cycles_on_device', False):
             # iterative refinement counts outer iterations of ir_inner_cycles V-cycles each
             self._cycles_host = int(self.device.fetch(self._counters[0])) * self._cycle_factor
+            self.check_waits()
             self._cycles_on_device = False
             self._iterations_host = self._cycles_host // self._cycle_factor * self._sweeps_per_cycle
         return self._cycles_host
@@ -151,7 +154,9 @@ class SolidMultigridProjector(SolidPressureProjector):
 
     def total_cycles(self):
         """V-cycles (or PCG iterations) of every solve so far (one readback)."""
-        return self._host_total + int(self.device.fetch(self._counters[1])) * self._cycle_factor
+        total = self._host_total + int(self.device.fetch(self._counters[1])) * self._cycle_factor
+        self.check_waits()
+        return total
 
     def _shapes(self):
         """Level shapes the grid allows (halving while all dims are even and >= 8)."""
@@ -226,6 +231,9 @@ class SolidMultigridProjector(SolidPressureProjector):
                     with dev.ordered():
                         workspace = torch.zeros(plan.workspace_bytes, dtype=torch.uint8, device=dev.device)
                     plan.workspace = workspace.data_ptr()
+                    if self._alarm is None:
+                        self._alarm = Alarm()
+                    plan.alarm = self._alarm.address
                     N.check(dev.lib.ffx_graph_plan_upload(C.byref(plan), dev.s))
                     entry = (plan, workspace)
             self._residents[first] = entry
@@ -574,6 +582,7 @@ class SolidMultigridProjector(SolidPressureProjector):
 
     def _solve(self, dt, previous_dt):
         s = self.settings
+        self.check_waits()
         self.last_cycles = 0
         if len(self.levels) == 1:
             return super().solve_pressure(dt, previous_dt)
@@ -658,6 +667,15 @@ class SolidMultigridProjector(SolidPressureProjector):
             self.last_iterations = budget * self._sweeps_per_cycle
             self._host_total += budget
         return True
+
+    def check_waits(self):
+        super().check_waits()
+        if self._alarm is not None:
+            def reset():
+                for entry in self._residents.values():
+                    if entry is not None:
+                        N.check(self.device.lib.ffx_graph_plan_reset(C.byref(entry[0]), self.device.s))
+            self._alarm.check(self.device, reset)
 
     def resident_timeouts(self):
         """Waits of resident solves that gave up (0 unless the GPU was held up for seconds)."""

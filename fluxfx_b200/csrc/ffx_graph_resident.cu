@@ -316,6 +316,7 @@ int ffx_graph_plan_upload(FfxGraphPlan* P, void* stream) {
     const gres::Candidate c = {P->tile[0], P->tile[1], P->blocks, 0.0};
     char* base = reinterpret_cast<char*>(P->workspace);
     P->shared_bytes = gres::fill(S, P->tail, c, 0, reinterpret_cast<gres::u64*>(base + kDomainBytes), D);
+    D.alarm = P->alarm;
     FFX_REQUIRE(D.blocks == P->blocks && P->shared_bytes <= resident::kSmem, "ffx_graph_plan_upload: not a plan that fits");
     cudaStream_t st = as_stream(stream);
     cudaError_t e = cudaMemcpyAsync(base, &D, sizeof D, cudaMemcpyHostToDevice, st);
@@ -342,6 +343,14 @@ int ffx_graph_solve(const FfxGraphPlan* P, float* p, const float* rhs, int32_t c
     A.aligned = ((uintptr_t)p | (uintptr_t)rhs) % 16 == 0;
     return gres::launch(whole, reinterpret_cast<const gres::Domain*>(P->workspace), 1, P->blocks, P->shared_bytes, A,
                         as_stream(stream));
+}
+
+int ffx_graph_plan_reset(const FfxGraphPlan* P, void* stream) {
+    FFX_REQUIRE(P, "ffx_graph_plan_reset: invalid arguments");
+    if (!P->workspace || P->blocks == 0) return FFX_OK;
+    return cuda_status(cudaMemsetAsync(reinterpret_cast<char*>(P->workspace) + kDomainBytes, 0,
+                                       (size_t)(P->workspace_bytes - kDomainBytes), as_stream(stream)),
+                       "ffx_graph_plan_reset");
 }
 
 int ffx_graph_plan_timeouts(const FfxGraphPlan* P, int32_t* count, void* stream) {

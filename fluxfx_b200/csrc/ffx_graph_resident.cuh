@@ -40,6 +40,7 @@ using resident::quotient;
 using resident::rim_items;
 using resident::u64;
 using resident::View;
+using resident::Waits;
 using resident::zero4;
 
 constexpr int kLevels = 10;
@@ -67,9 +68,10 @@ struct Domain {
     const double* inverse;             // dense FP64 inverse of the coarsest level, or NULL
     u64* ws;
     int64_t tail_rhs, tail_p, maxima, control;   // words
-    unsigned* epochs;                  // two per block: exchange and tail numbers reached
+    unsigned* epochs;                  // two per block: the next launch's exchanges and decisions count from them
     int exchanges;                     // of a cycle's sweeps, all levels in tiles
     unsigned* timeouts;
+    int* alarm;
     int tile_f4, tail_f4;
     double tol;
     int max_cycles;
@@ -318,7 +320,7 @@ __device__ __forceinline__ void relax(GView& g, int level, const float2* table, 
             }
         }
         if (ex.on) {
-            collect(v.ll + half, from, two ? v.Q : v.P, dst, ex.epoch, ex.dead, ex.timeouts);
+            collect(v.ll + half, from, two ? v.Q : v.P, dst, ex.epoch, ex.waits);
             ex.turn ^= 1u << level;
             ++ex.epoch;
         }
@@ -467,10 +469,9 @@ __device__ __forceinline__ float domain_max(const Domain& D, float mine, int til
                 break;
             }
             if ((spin & 255) == 255) {
-                if (*ex.dead) break;
+                if (ex.waits.over()) break;
                 if (spin >= resident::kSpinLimit) {
-                    *ex.dead = 1;
-                    atomicAdd(ex.timeouts, 1u);
+                    ex.waits.give_up();
                     break;
                 }
             }
@@ -488,10 +489,10 @@ __device__ __forceinline__ float domain_max(const Domain& D, float mine, int til
 }
 
 // ------------------------------------------------------------------- roles
-__device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4* smem, volatile int* dead,
+__device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4* smem, const Waits& waits,
                                          int block) {
     const int tid = threadIdx.x;
-    Exchange none = {false, 0u, 0u, dead, D.timeouts};
+    Exchange none = {false, 0u, 0u, waits};
     unsigned flip = 0;
     auto view = [&](int k) { return make_gview(D, D.tv[k], 0, 0, smem, nullptr, flip >> k & 1u); };
     const int first = D.dist, last = D.count - 1;
@@ -516,8 +517,7 @@ __device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4*
                     break;
                 }
                 if ((spin & 255) == 255 && spin >= resident::kSpinLimit) {
-                    *dead = 1;
-                    atomicAdd(D.timeouts, 1u);
+                    waits.give_up();
                     break;
                 }
             }
@@ -532,7 +532,7 @@ __device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4*
                 from[u] = s < slots ? 4 * s : -1;
                 dst[u] = s;
             }
-            collect(D.ws + D.tail_rhs, from, top.v.R, dst, number, dead, D.timeouts);
+            collect(D.ws + D.tail_rhs, from, top.v.R, dst, number, waits);
         }
         __syncthreads();
         for (int k = first; k <= last; ++k) {
@@ -579,13 +579,13 @@ __device__ __forceinline__ void run_tail(const Domain& D, const Call& A, float4*
 // coarse level and one V-cycle from zero runs (the coarse part of a cycle).
 template <bool LINKS>
 __device__ __forceinline__ void run_tile(const Domain& D, const Call& A, float4* smem, float2* table, float* scratch,
-                                         volatile int* dead, int tile) {
+                                         const Waits& waits, int tile) {
     const int tid = threadIdx.x;
     const int by = tile % D.gy, bz = tile / D.gy;
     unsigned flip = 0;
     auto view = [&](int k) { return make_gview(D, D.lv[k], by, bz, smem, D.ws, flip >> k & 1u); };
     const unsigned ex_base = D.epochs[2 * tile], base = D.epochs[2 * tile + 1];
-    Exchange ex = {true, ex_base + 1u, 0u, dead, D.timeouts};
+    Exchange ex = {true, ex_base + 1u, 0u, waits};
     unsigned number = base, turn = 0;
     float* const P_out = A.batched ? D.p : A.p;
     const float* const rhs = A.batched ? D.rhs : A.rhs;
@@ -731,7 +731,7 @@ __device__ __forceinline__ void run_tile(const Domain& D, const Call& A, float4*
                     from[u] = in ? published(v, x, gy, gz) : -1;
                     dst[u] = s;
                 }
-                collect(D.ws + D.tail_p, from, v.P, dst, number, dead, D.timeouts);
+                collect(D.ws + D.tail_p, from, v.P, dst, number, waits);
             }
             __syncthreads();
         }
@@ -809,8 +809,9 @@ __global__ void __launch_bounds__(kThreads, 1) graph_resident_kernel(const Domai
     const int clear = tail ? D.tail_f4 : D.tile_f4;
     for (int i = tid; i < clear; i += kThreads) smem[i] = zero4();
     __syncthreads();
-    if (tail) run_tail(D, A, smem, &dead, block);
-    else run_tile<LINKS>(D, A, smem, table, scratch, &dead, block);
+    const Waits waits = {&dead, D.timeouts, D.alarm};
+    if (tail) run_tail(D, A, smem, waits, block);
+    else run_tile<LINKS>(D, A, smem, table, scratch, waits, block);
 }
 
 }  // namespace gres

@@ -744,6 +744,7 @@ int run_resident(const FfxRelaxPlan& P, int cycles, float dt, bool from_zero, fl
     A.ws = reinterpret_cast<resident::u64*>(P.workspace);
     A.epochs = reinterpret_cast<unsigned*>(A.ws);
     A.timeouts = A.epochs + 2 * kHeaderWords - 1;
+    A.alarm = P.alarm;
     const int fit = tile_fit(P, dist, P.tile[0], P.tile[1]);
     FFX_REQUIRE(fit >= 0 && A.gy * A.gz < kHeaderWords * 2 - 2, "resident tile out of range");
     const bool one = fit == 1;
@@ -930,6 +931,13 @@ int ffx_relax_cycles(const FfxRelaxPlan* P, int32_t cycles, float dt, int32_t fr
     }
     *swapped = cur[0] != p0;
     return FFX_OK;
+}
+
+int ffx_relax_reset(const FfxRelaxPlan* P, void* stream) {
+    FFX_REQUIRE(P, "ffx_relax_reset: invalid arguments");
+    if (!P->workspace || P->workspace_bytes == 0) return FFX_OK;
+    return cuda_status(cudaMemsetAsync(P->workspace, 0, (size_t)P->workspace_bytes, as_stream(stream)),
+                       "ffx_relax_reset");
 }
 
 int ffx_relax_timeouts(const FfxRelaxPlan* P, int32_t* count, void* stream) {

@@ -26,7 +26,7 @@
 //
 // Blocks wait for one another, so the launch is cooperative (all blocks
 // resident at once); every wait is bounded: after kSpinLimit polls a block
-// stops waiting, counts a timeout and runs to its end.
+// stops waiting, counts a timeout, tells the host (Waits) and runs to its end.
 #pragma once
 #include "ffx_host.cuh"
 
@@ -68,6 +68,7 @@ struct Params {
     unsigned* epochs;            // exchange number reached, per block
     unsigned epochs_used;        // exchanges a launch may number
     unsigned* timeouts;
+    int* alarm;                  // host memory, or NULL (Waits)
     int tile_f4, tail_f4;        // float4 of shared memory to clear, by role
     Level lv[kLevels];           // tiles: levels 0 .. dist (dist: the tail's level, its pressure only)
     Level tv[kLevels];           // tail: levels dist .. count - 1
@@ -177,11 +178,24 @@ __device__ __forceinline__ bool get4(const u64* from, unsigned epoch, float4& v)
            (unsigned)(d >> 32) == epoch;
 }
 
+// The bounded waits of a block: once one has given up the others no longer wait, the
+// device's count goes up and the word that the host watches is set.
+struct Waits {
+    volatile int* dead;
+    unsigned* timeouts;
+    int* alarm;
+    __device__ __forceinline__ bool over() const { return *dead != 0; }
+    __device__ __forceinline__ void give_up() const {
+        *dead = 1;
+        atomicAdd(timeouts, 1u);
+        if (alarm) atomicExch_system(alarm, 1);
+    }
+};
+
 // One bounded poll loop over up to kRimItems float4 of a thread: words
 // `base + from[u]` (from[u] < 0: none) into `to + dst[u]`.
 __device__ __forceinline__ void collect(const u64* base, const int (&from)[kRimItems], float4* to,
-                                        const int (&dst)[kRimItems], unsigned epoch, volatile int* dead,
-                                        unsigned* timeouts) {
+                                        const int (&dst)[kRimItems], unsigned epoch, const Waits& waits) {
     unsigned pending = 0;
 #pragma unroll
     for (int u = 0; u < kRimItems; ++u) pending |= from[u] >= 0 ? 1u << u : 0u;
@@ -195,10 +209,9 @@ __device__ __forceinline__ void collect(const u64* base, const int (&from)[kRimI
             }
         }
         if ((spin & 255) == 255 && pending) {
-            if (*dead) return;
+            if (waits.over()) return;
             if (spin >= kSpinLimit) {
-                *dead = 1;
-                atomicAdd(timeouts, 1u);
+                waits.give_up();
                 return;
             }
         }
@@ -210,8 +223,7 @@ struct Exchange {
     bool on;
     unsigned epoch;      // of the next exchange
     unsigned turn;       // bit k: which of level k's two published copies comes next
-    volatile int* dead;
-    unsigned* timeouts;
+    Waits waits;
 };
 
 // Words of row (gy, gz)'s float4 x in a level's published rows.
@@ -343,7 +355,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             }
         }
         if (ex.on) {
-            collect(v.ll + half, from, ONE ? v.P : v.Q, dst, ex.epoch, ex.dead, ex.timeouts);
+            collect(v.ll + half, from, ONE ? v.P : v.Q, dst, ex.epoch, ex.waits);
             ex.turn ^= 1u << level;
             ++ex.epoch;
         }
@@ -476,10 +488,10 @@ __device__ __forceinline__ void separable_solve(const View& v, double* wk, const
 
 // ------------------------------------------------------------------- roles
 // A block with whole levels (the tail, or everything when dist = 0).
-__device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (*kd)[28], volatile int* dead,
+__device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (*kd)[28], const Waits& waits,
                                          unsigned base) {
     const int tid = threadIdx.x;
-    Exchange none = {false, 0u, 0u, dead, A.timeouts};
+    Exchange none = {false, 0u, 0u, waits};
     unsigned flip = 0;       // bit k: level k's pressure is in its second copy
     auto view = [&](int k) { return make_view(A.tv[k], 0, 0, smem, nullptr, flip >> k & 1u); };
     auto smooth = [&](View& v, int k, bool zero, int count) {
@@ -512,7 +524,7 @@ __device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (
                     from[u] = s < slots ? 4 * s : -1;
                     dst[u] = s;
                 }
-                collect(A.ws + A.tail_rhs, from, top.R, dst, epoch, dead, A.timeouts);
+                collect(A.ws + A.tail_rhs, from, top.R, dst, epoch, waits);
             }
             __syncthreads();
         }
@@ -560,13 +572,13 @@ __device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (
 
 // A block with a tile of the levels 0 .. dist - 1.
 template <bool MASK, bool ONE>
-__device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (*kd)[28], volatile int* dead,
+__device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (*kd)[28], const Waits& waits,
                                          unsigned base) {
     const int tid = threadIdx.x;
     const int by = blockIdx.x % A.gy, bz = blockIdx.x / A.gy;
     unsigned flip = 0;
     auto view = [&](int k) { return make_view(A.lv[k], by, bz, smem, A.ws, flip >> k & 1u); };
-    Exchange ex = {true, base + 1u, 0u, dead, A.timeouts};
+    Exchange ex = {true, base + 1u, 0u, waits};
     unsigned* cls = reinterpret_cast<unsigned*>(smem + A.cls_off);
     auto smooth = [&](View& v, int k, bool zero, int count) {
         if (k == 0) {
@@ -670,7 +682,7 @@ __device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (
                     from[u] = in ? published(g, x, gy, gz) : -1;
                     dst[u] = s;
                 }
-                collect(A.ws + A.tail_p, from, g.P, dst, epoch, dead, A.timeouts);
+                collect(A.ws + A.tail_p, from, g.P, dst, epoch, waits);
             }
             __syncthreads();
         }
@@ -717,8 +729,9 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
     }
     __syncthreads();
     const unsigned base = A.dist ? A.epochs[blockIdx.x] : 0u;
-    if (tail) run_tail(A, smem, kd, &dead, base);
-    else run_tile<MASK, ONE>(A, smem, kd, &dead, base);
+    const Waits waits = {&dead, A.timeouts, A.alarm};
+    if (tail) run_tail(A, smem, kd, waits, base);
+    else run_tile<MASK, ONE>(A, smem, kd, waits, base);
     __syncthreads();
     if (tid == 0 && A.dist) A.epochs[blockIdx.x] = base + A.epochs_used;
 }

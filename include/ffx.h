@@ -398,6 +398,8 @@ typedef struct FfxRelaxPlan {
     int64_t workspace_bytes;  /* filled */
     void* workspace;          /* caller's, 16-byte aligned, zeroed once; for one solve at a time */
     FfxRelaxLevel level[FFX_RELAX_LEVELS];
+    int32_t* alarm;           /* NULL, or a word of host memory that the device writes (pinned): set to 1 when
+                               * a bounded wait of a solve gives up, after which its pressure is wrong */
 } FfxRelaxPlan;
 /* Fills the plan for its grids (host only). Whether classes is NULL matters here. */
 int ffx_relax_plan(FfxRelaxPlan* plan);
@@ -409,6 +411,8 @@ int ffx_relax_cycles(const FfxRelaxPlan* plan, int32_t cycles, float dt, int32_t
 /* Bounded waits of resident solves that gave up, since the workspace was zeroed
  * (waits for the stream). Anything but 0 means wrong pressures. */
 int ffx_relax_timeouts(const FfxRelaxPlan* plan, int32_t* count, void* stream);
+/* Zeroes the workspace again (on the stream), after a wait that gave up. */
+int ffx_relax_reset(const FfxRelaxPlan* plan, void* stream);
 /* One byte per cell: open neighbours cx + 3 cy + 9 cz along the axes, 27 in a
  * solid; rows padded to a multiple of four bytes (with 27), so `classes` holds
  * 4 ceil(nx / 4) * ny * nz bytes and starts on 4. */
@@ -481,6 +485,7 @@ typedef struct FfxGraphPlan {
     int32_t shared_bytes;     /* filled by ffx_graph_plan_upload */
     int64_t workspace_bytes;
     void* workspace;          /* caller's, 256-byte aligned, zeroed once; for one solve at a time */
+    int32_t* alarm;           /* as in FfxRelaxPlan; before ffx_graph_plan_upload */
 } FfxGraphPlan;
 /* Whether and how the hierarchy fits (host only; blocks = 0 when it does not). */
 int ffx_graph_plan(FfxGraphPlan* plan);
@@ -494,6 +499,8 @@ int ffx_graph_solve(const FfxGraphPlan* plan, float* p, const float* rhs, int32_
                     double tol, int32_t max_cycles, int32_t* counters, void* stream);
 /* Bounded waits that gave up since the workspace was zeroed (waits for the stream). */
 int ffx_graph_plan_timeouts(const FfxGraphPlan* plan, int32_t* count, void* stream);
+/* Zeroes the plan's numbers, words and count again (on the stream), after a wait that gave up. */
+int ffx_graph_plan_reset(const FfxGraphPlan* plan, void* stream);
 
 /* Level-0 link bytes from the mask: bit 2a / 2a+1 = the face to the lower /
  * upper neighbour along axis a joins two fluid cells inside the domain, bit 6
