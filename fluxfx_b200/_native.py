@@ -69,7 +69,7 @@ class FfxGraphPlan(C.Structure):
     _fields_ = [('count', i32), ('pre0', i32), ('post0', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32),
                 ('omega', f32), ('inverse', vp), ('level', FfxGraphLevel * GRAPH_PLAN_LEVELS), ('blocks', i32),
                 ('tile', i32 * 2), ('tail', i32), ('shared_bytes', i32), ('workspace_bytes', i64), ('workspace', vp),
-                ('alarm', vp)]
+                ('alarm', vp), ('sms', i32)]
 
 
 TAIL_LEVELS = 8
@@ -104,7 +104,7 @@ class FfxRelaxLevel(C.Structure):
 class FfxRelaxPlan(C.Structure):
     _fields_ = [('count', i32), ('pre', i32), ('post', i32), ('last_sweeps', i32), ('tail', i32), ('tile', i32 * 2),
                 ('omega', f32), ('basis', vp), ('classes', vp), ('workspace_bytes', i64), ('workspace', vp),
-                ('level', FfxRelaxLevel * RELAX_LEVELS), ('alarm', vp)]
+                ('level', FfxRelaxLevel * RELAX_LEVELS), ('alarm', vp), ('sms', i32)]
 
 
 class FfxBrickStats(C.Structure):

@@ -46,11 +46,12 @@ class Alarm:
 
 
 class Relaxation:
-    def __init__(self, device, shapes, extent, omega, *, pre=1, post=1, last=1, basis=None, classes=None):
+    def __init__(self, device, shapes, extent, omega, *, pre=1, post=1, last=1, basis=None, classes=None, sms=0):
         self.device = device
         self._keep = (basis, classes)
         plan = self.plan = N.FfxRelaxPlan()
         plan.count, plan.pre, plan.post, plan.last_sweeps, plan.omega = len(shapes), pre, post, last, omega
+        plan.sms = sms
         plan.basis = basis.data_ptr() if basis is not None else None
         plan.classes = classes.data_ptr() if classes is not None else None
         for slot, shape in zip(plan.level, shapes):

@@ -553,7 +553,7 @@ bool plan_resident(Builder& B, int first) {
     }
     std::vector<gres::Candidate> chosen;
     std::vector<int> dist;
-    if (!gres::plan_blocks(specs.data(), P.count, chosen, dist)) return false;
+    if (!gres::plan_blocks(specs.data(), P.count, resident_sms(), chosen, dist)) return false;
     P.resident_first = first;
     P.resident_domains = B.reserve(sizeof(gres::Domain) * P.count);
     P.resident_blocks = P.resident_smem = 0;

@@ -26,9 +26,9 @@ struct Candidate {
     double cost;
 };
 
-// Tiles for every domain so that all blocks of all domains are resident at
-// once; false when they do not fit. dist: levels in tiles, per domain.
-bool plan_blocks(const Spec* specs, int count, std::vector<Candidate>& chosen, std::vector<int>& dist);
+// Tiles for every domain so that all blocks of all domains are resident on `sms`
+// SMs at once; false when they do not fit. dist: levels in tiles, per domain.
+bool plan_blocks(const Spec* specs, int count, int sms, std::vector<Candidate>& chosen, std::vector<int>& dist);
 // 64-bit words of a domain's published rows and header.
 int64_t words_of(const Spec& S, int dist, const Candidate& c);
 // The domain's record; returns the bytes of shared memory its blocks need.

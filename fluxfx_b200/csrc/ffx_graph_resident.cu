@@ -13,8 +13,6 @@ namespace ffx {
 namespace gres {
 namespace {
 
-constexpr int kSms = 148;
-
 int up4(int v) { return (v + 3) & ~3; }
 int x4_of(const FfxGraphLevel& g) { return up4(g.nx) / 4; }
 int64_t slots_of(const FfxGraphLevel& g) { return (int64_t)x4_of(g) * g.ny * g.nz; }
@@ -50,7 +48,7 @@ int tile_f4(const Spec& S, int dist, int ty, int tz, bool two) {
 
 }  // namespace
 
-bool candidates(const Spec& S, std::vector<Candidate>& out, int& dist) {
+bool candidates(const Spec& S, int sms, std::vector<Candidate>& out, int& dist) {
     out.clear();
     if (S.count < 1 || S.count > kLevels || (S.whole && S.count < 2)) return false;
     // the tail: levels that one block holds, never level 0
@@ -65,7 +63,7 @@ bool candidates(const Spec& S, std::vector<Candidate>& out, int& dist) {
     const bool tail = dist < S.count;
     if (S.inverse && !tail) return false;
     const FfxGraphLevel& g = S.level[0];
-    const int align = 1 << (tail ? dist : dist - 1), cap = kSms - (tail ? 1 : 0), x4 = x4_of(g);
+    const int align = 1 << (tail ? dist : dist - 1), cap = sms - (tail ? 1 : 0), x4 = x4_of(g);
     for (int ty = align; ty < g.ny + align; ty += align)
         for (int tz = align; tz < g.nz + align; tz += align) {
             const int tiles = ((g.ny + ty - 1) / ty) * ((g.nz + tz - 1) / tz);
@@ -79,13 +77,13 @@ bool candidates(const Spec& S, std::vector<Candidate>& out, int& dist) {
     return !out.empty();
 }
 
-bool plan_blocks(const Spec* specs, int count, std::vector<Candidate>& chosen, std::vector<int>& dist) {
+bool plan_blocks(const Spec* specs, int count, int sms, std::vector<Candidate>& chosen, std::vector<int>& dist) {
     std::vector<std::vector<Candidate>> all(count);
     chosen.assign(count, Candidate{});
     dist.assign(count, 0);
     int used = 0;
     for (int d = 0; d < count; ++d) {
-        if (!candidates(specs[d], all[d], dist[d])) return false;
+        if (!candidates(specs[d], sms, all[d], dist[d])) return false;
         // the fewest blocks that hold it, of those the least work
         std::sort(all[d].begin(), all[d].end(), [](const Candidate& a, const Candidate& b) {
             return a.blocks != b.blocks ? a.blocks < b.blocks : a.cost < b.cost;
@@ -93,7 +91,7 @@ bool plan_blocks(const Spec* specs, int count, std::vector<Candidate>& chosen, s
         chosen[d] = all[d][0];
         used += chosen[d].blocks;
     }
-    if (used > kSms) return false;
+    if (used > sms) return false;
     // then blocks to whichever domain takes longest, while there are any
     for (;;) {
         int worst = 0;
@@ -101,7 +99,7 @@ bool plan_blocks(const Spec* specs, int count, std::vector<Candidate>& chosen, s
             if (chosen[d].cost > chosen[worst].cost) worst = d;
         const Candidate* next = nullptr;
         for (const Candidate& c : all[worst])
-            if (c.cost < chosen[worst].cost && used - chosen[worst].blocks + c.blocks <= kSms &&
+            if (c.cost < chosen[worst].cost && used - chosen[worst].blocks + c.blocks <= sms &&
                 (!next || c.blocks < next->blocks || (c.blocks == next->blocks && c.cost < next->cost)))
                 next = &c;
         if (!next) return true;
@@ -217,23 +215,18 @@ int fill(const Spec& S, int dist, const Candidate& c, int first_block, u64* ws, 
 
 int launch(bool links, const Domain* domains, int count, int blocks, int smem, const Call& A, cudaStream_t st) {
     static std::atomic<uint64_t> ready{0};
-    static std::atomic<int> sms{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_status(e, "cudaGetDevice");
     if (!(ready.load(std::memory_order_acquire) >> (dev & 63) & 1)) {
-        int coop = 0, n = 0;
-        e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(graph_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, resident::kSmem);
+        e = cudaFuncSetAttribute(graph_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, resident::kSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(graph_resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, resident::kSmem);
         if (e != cudaSuccess) return cuda_status(e, "graph_resident_kernel");
-        FFX_REQUIRE(coop && n >= kSms, "graph_resident_kernel: needs a cooperative launch over %d SMs", kSms);
-        sms.store(n, std::memory_order_relaxed);
         ready.fetch_or(uint64_t(1) << (dev & 63), std::memory_order_release);
     }
+    FFX_REQUIRE(blocks <= resident_sms(), "graph_resident_kernel: planned for %d SMs, the device has %d", blocks,
+                resident_sms());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(kThreads);
@@ -298,7 +291,8 @@ int ffx_graph_plan(FfxGraphPlan* P) {
     P->workspace_bytes = 0;
     std::vector<gres::Candidate> c;
     std::vector<int> dist;
-    if (!gres::plan_blocks(&S, 1, c, dist)) return FFX_OK;      // it does not fit: blocks stays 0
+    P->sms = P->sms > 0 ? std::min(P->sms, resident_sms()) : resident_sms();
+    if (!gres::plan_blocks(&S, 1, P->sms, c, dist)) return FFX_OK;      // it does not fit: blocks stays 0
     P->blocks = c[0].blocks;
     P->tile[0] = c[0].ty;
     P->tile[1] = c[0].tz;

@@ -60,6 +60,12 @@ inline int launch_pdl(const char* what, void (*kernel)(KArgs...), dim3 grid, dim
     return launch_status(what);
 }
 
+// Blocks of one per SM that a cooperative launch can keep on the current device at
+// once: its SMs, at most the 148 of a whole chip, which plans are laid out for; 1
+// where there are no cooperative launches. 148 where no device answers (planning
+// on a machine without one).
+int resident_sms();
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Extents within [2^-18, 2^30]: with at most 4096 cells per axis every

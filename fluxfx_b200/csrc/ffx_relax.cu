@@ -571,7 +571,6 @@ using resident::Level;
 using resident::Params;
 
 constexpr int kHeaderWords = 128;      // exchange numbers of the blocks, the timeout counter
-constexpr int kSms = 148;
 
 int64_t slots_of(const int32_t n[3]) { return (int64_t)(up4(n[0]) / 4) * n[1] * n[2]; }
 
@@ -611,13 +610,13 @@ int tile_fit(const FfxRelaxPlan& P, int dist, int ty, int tz) {
 }
 
 // Tiles of rows for the levels above the tail: as few cells per block as the
-// SMs allow, then as small a rim. Tile edges are multiples of 2^levels, so a
+// plan's SMs allow, then as small a rim. Tile edges are multiples of 2^levels, so a
 // tile restricts into its own coarse tile. False when the grid does not fit.
 bool plan_tiles(FfxRelaxPlan& P) {
     const int dist = P.tail;
     const bool tail = dist < P.count;
     const int32_t* n = P.level[0].grid.n;
-    const int align = 1 << (tail ? dist : dist - 1), cap = kSms - (tail ? 1 : 0);
+    const int align = 1 << (tail ? dist : dist - 1), cap = P.sms - (tail ? 1 : 0);
     double best = 1e300;
     for (int ty = align; ty < n[1] + align; ty += align)
         for (int tz = align; tz < n[2] + align; tz += align) {
@@ -789,23 +788,6 @@ int run_resident(const FfxRelaxPlan& P, int cycles, float dt, bool from_zero, fl
                : launch_resident<false, false>(A, blocks, smem, st);
 }
 
-// Whether this device takes the cooperative launch of a plan made for 148 SMs.
-bool cooperative_device() {
-    static std::atomic<int> known[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    std::atomic<int>& slot = known[dev & 63];
-    int v = slot.load(std::memory_order_acquire);
-    if (v == 0) {
-        int coop = 0, sms = 0;
-        const bool ok = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess &&
-                        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
-        v = ok && coop && sms >= kSms ? 1 : 2;
-        slot.store(v, std::memory_order_release);
-    }
-    return v == 1;
-}
-
 }  // namespace
 }  // namespace ffx
 
@@ -835,6 +817,7 @@ int ffx_relax_plan(FfxRelaxPlan* P) {
     FFX_REQUIRE(!P->basis || P->tail < P->count, "ffx_relax_plan: no block holds the coarsest level");
     P->tile[0] = P->tile[1] = 0;
     P->workspace_bytes = 0;
+    P->sms = P->sms > 0 ? std::min(P->sms, resident_sms()) : resident_sms();
     if (P->tail == 0) return FFX_OK;
     if (plan_tiles(*P)) {
         P->workspace_bytes = 8 * published_words(*P);
@@ -878,7 +861,8 @@ int ffx_relax_cycles(const FfxRelaxPlan* P, int32_t cycles, float dt, int32_t fr
         return run_one_block(*P, 0, cycles, dt, from_zero ? nullptr : p0, P->level[0].rhs, p0, st);
     if (fits) {
         FFX_REQUIRE(P->workspace && (uintptr_t)P->workspace % 16 == 0, "ffx_relax_cycles: workspace missing");
-        FFX_REQUIRE(cooperative_device(), "ffx_relax_cycles: needs a cooperative launch over 148 SMs");
+        FFX_REQUIRE(resident_sms() >= P->sms, "ffx_relax_cycles: planned for %d SMs, the device has %d", P->sms,
+                    resident_sms());
         return run_resident(*P, cycles, dt, from_zero != 0, p0, st);
     }
     float* cur[FFX_RELAX_LEVELS];

@@ -1,5 +1,7 @@
 // Runtime entry points: error text, device query and probe, seeds, collider
 // masks and reductions.
+#include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "ffx_host.cuh"
@@ -13,6 +15,29 @@ std::string& last_error_buffer() {
 }
 
 int g_pdl = 1;
+
+int resident_sms() {
+    constexpr int kChip = 148;
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return kChip;
+    }
+    std::atomic<int>& slot = known[dev & 63];
+    int v = slot.load(std::memory_order_acquire);
+    if (v == 0) {
+        int coop = 0, sms = 0;
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return kChip;
+        }
+        v = coop ? std::min(sms, kChip) : 1;
+        slot.store(v, std::memory_order_release);
+    }
+    return v;
+}
 
 namespace {
 

@@ -400,8 +400,11 @@ typedef struct FfxRelaxPlan {
     FfxRelaxLevel level[FFX_RELAX_LEVELS];
     int32_t* alarm;           /* NULL, or a word of host memory that the device writes (pinned): set to 1 when
                                * a bounded wait of a solve gives up, after which its pressure is wrong */
+    int32_t sms;              /* SMs that a resident solve may use; 0: all of the current device, which is
+                               * filled in (one, where it has no cooperative launches) */
 } FfxRelaxPlan;
-/* Fills the plan for its grids (host only). Whether classes is NULL matters here. */
+/* Fills the plan for its grids (host only). Whether classes is NULL matters here. A
+ * grid that does not fit the SMs is not resident. */
 int ffx_relax_plan(FfxRelaxPlan* plan);
 /* `cycles` V-cycles on L p = rhs / dt; with one level, `cycles` times last_sweeps
  * weighted Jacobi sweeps. from_zero: the iterate starts from zero and level 0's
@@ -486,6 +489,7 @@ typedef struct FfxGraphPlan {
     int64_t workspace_bytes;
     void* workspace;          /* caller's, 256-byte aligned, zeroed once; for one solve at a time */
     int32_t* alarm;           /* as in FfxRelaxPlan; before ffx_graph_plan_upload */
+    int32_t sms;              /* as in FfxRelaxPlan; before ffx_graph_plan */
 } FfxGraphPlan;
 /* Whether and how the hierarchy fits (host only; blocks = 0 when it does not). */
 int ffx_graph_plan(FfxGraphPlan* plan);
