@@ -85,7 +85,9 @@ class BatchedSmoke:
             self._fill(self._domains[i], s, src, cell, cfl, dt_max, dt0)
         need = C.c_int64(0)
         N.check(self.lib.ffx_batch_workspace_bytes(self._domains, len(solvers), C.byref(need)))
-        self.workspace = torch.zeros(int(need.value) + 256, dtype=torch.uint8, device=self.device.device)
+        with self.device.ordered():
+            self.workspace = torch.zeros(int(need.value) + 256, dtype=torch.uint8, device=self.device.device)
+        self.device.synchronize()       # the plan is written from the default stream
         base = (self.workspace.data_ptr() + 255) & ~255
         plan = C.c_void_p()
         N.check(self.lib.ffx_batch_create(self._domains, len(solvers), C.c_void_p(base), int(need.value),

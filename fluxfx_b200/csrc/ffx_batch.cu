@@ -821,6 +821,9 @@ int ffx_batch_create(const FfxBatchDomain* domains, int32_t count, void* workspa
     // no word carries the number of an exchange to come
     if (!e && P->resident_bytes > 0)
         e = cuda_status(cudaMemset(P->ws + P->resident_words, 0, (size_t)P->resident_bytes), "ffx_batch_create: words");
+    // neither the copy nor the clearing waits for the device, and the steps run on
+    // streams that need not wait for the default one
+    if (!e) e = cuda_status(cudaStreamSynchronize(cudaStreamLegacy), "ffx_batch_create: upload");
     if (e) {
         delete P;
         return e;
