@@ -51,12 +51,13 @@ class MultigridPressureProjector(PressureProjector):
         self.prolong_kernel = KernelHandle('mg_prolong.glsl')
         dev = self.device
         for i, shape in enumerate(shapes):
+            # (fields below level 0: made for the first cycle of separate passes)
             self.levels.append({
                 'shape': shape, 'inv': tuple(n / e for n, e in zip(shape, grid.extent)),
-                'p': self.pressure if i == 0 else dev.texture(shape) if self._separate_passes else None,
-                'q': self.spare if i == 0 else dev.texture(shape) if self._separate_passes else None,
-                'rhs': self.before if i == 0 else dev.texture(shape) if self._separate_passes else None,
-                'residual': None})
+                'p': self.pressure if i == 0 else None, 'q': self.spare if i == 0 else None,
+                'rhs': self.before if i == 0 else None, 'residual': None})
+        if self._separate_passes:
+            self._make_fields()
         coarsest = shapes[-1]
         if len(shapes) > 1 and s.coarse_solver == 'DIRECT' and (
                 coarsest == (4, 4, 4) or (s.mg_max_levels and prod(coarsest) <= MAX_DIRECT_CELLS)):
@@ -67,20 +68,36 @@ class MultigridPressureProjector(PressureProjector):
             self.coarse_basis = torch.as_tensor(neumann_basis(coarsest, grid.extent)).to(dev.device)
         self.pre_sweeps = s.mg_pre_sweeps or 3
         self.post_sweeps = s.mg_post_sweeps or 3
-        # the levels below the first live inside the native cycles
-        self._relaxation = Relaxation(dev, shapes, grid.extent, 2.0 / 3.0, pre=self.pre_sweeps, post=self.post_sweeps,
-                                      last=80, basis=self.coarse_basis) if (
-            len(shapes) > 1 and not self._separate_passes) else None
-        self._cycle_sweeps = (len(shapes) - 1) * (self.pre_sweeps + self.post_sweeps) + (
-            0 if self.coarse_basis is not None else 80)
+        self._relaxation = None
+        self._whole_cycles()
         self.last_cycles = 0
         self.last_coarse_solves = 0
         self._rmax = torch.zeros(2, dtype=torch.float32, device=dev.device)
 
+    def _whole_cycles(self):
+        """The plan of native cycles (the levels below the first live inside them) for
+        the sweep counts as they are now, or None: one level, 16-bit storage, or a
+        side without sweeps."""
+        if len(self.levels) == 1 or self._separate_passes or min(self.pre_sweeps, self.post_sweeps) < 1:
+            return None
+        r = self._relaxation
+        if r is None or (r.plan.pre, r.plan.post) != (self.pre_sweeps, self.post_sweeps):
+            r = self._relaxation = Relaxation(
+                self.device, [v['shape'] for v in self.levels], self.grid.extent, 2.0 / 3.0, pre=self.pre_sweeps,
+                post=self.post_sweeps, last=80, basis=self.coarse_basis)
+        return r
+
+    def _make_fields(self):
+        for level in self.levels[1:]:
+            for name in ('p', 'q', 'rhs'):
+                if level[name] is None:
+                    level[name] = self.device.texture(level['shape'])
+
     @property
     def allocated_bytes(self):
-        extra = self._relaxation.allocated_bytes if self._relaxation is not None else 4 * sum(
-            3 * prod(v['shape']) for v in self.levels[1:])
+        extra = sum(4 * prod(v['shape']) for v in self.levels[1:] for name in ('p', 'q', 'rhs') if v[name] is not None)
+        if self._relaxation is not None:
+            extra += self._relaxation.allocated_bytes
         return super().allocated_bytes + extra + sum(
             8 * t.numel() for t in (self.coarse_matrix, self.coarse_basis) if t is not None)
 
@@ -104,15 +121,18 @@ class MultigridPressureProjector(PressureProjector):
             self.device.call('ffx_jacobi', self._n3(level), self._inv3(level), None, ptr(level['p']),
                              ptr(level['rhs']), dt, 2.0 / 3.0, ptr(level['q']), s)
             level['p'], level['q'] = level['q'], level['p']
+            self.last_iterations += 1
 
     def cycle(self, index, dt):
         """One V-cycle, a launch per pass."""
+        self._make_fields()
         level = self.levels[index]
         s = self.device.s
         if index == len(self.levels) - 1:
             if self.coarse_matrix is not None:
                 self.device.call('ffx_direct_solve', prod(level['shape']), ptr(self.coarse_matrix),
                                  ptr(level['rhs']), dt, ptr(level['p']), s)
+                self.last_coarse_solves += 1
             else:
                 self.smooth(level, dt, 80)
             return
@@ -129,20 +149,20 @@ class MultigridPressureProjector(PressureProjector):
     def _cycles(self, count, dt, from_zero=False):
         """``count`` V-cycles on level 0's iterate (not read when ``from_zero``)."""
         level = self.levels[0]
-        if self._separate_passes:
+        self.last_cycles += count
+        whole = self._whole_cycles()
+        if whole is None:
             if from_zero:
                 level['p'].zero_()
             for _ in range(count):
                 self.cycle(0, dt)
-        else:
-            self._relax(level, count, dt, from_zero)
-        self.last_cycles += count
-        self.last_iterations += count * self._cycle_sweeps
-        if self.coarse_basis is not None:
+            return
+        level['p'], level['q'] = whole.run(level['p'], level['q'], level['rhs'], count, dt, from_zero)
+        self.last_iterations += count * (len(self.levels) - 1) * (self.pre_sweeps + self.post_sweeps)
+        if self.coarse_matrix is not None:
             self.last_coarse_solves += count
-
-    def _relax(self, level, count, dt, from_zero):
-        level['p'], level['q'] = self._relaxation.run(level['p'], level['q'], level['rhs'], count, dt, from_zero)
+        else:
+            self.last_iterations += count * 80
 
     def check_waits(self):
         super().check_waits()
