@@ -218,7 +218,8 @@ class SolidMultigridProjector(SolidPressureProjector):
             plan = N.FfxGraphPlan()
             levels = self.levels[first:]
             entry = None
-            if 1 <= len(levels) <= N.GRAPH_PLAN_LEVELS and (first > 0 or len(levels) > 1):
+            sweeps = (self.coarse_pre, self.coarse_post) + ((self.pre_sweeps, self.post_sweeps) if first == 0 else ())
+            if 1 <= len(levels) <= N.GRAPH_PLAN_LEVELS and (first > 0 or len(levels) > 1) and min(sweeps) > 0:
                 plan.count = len(levels)
                 plan.pre, plan.post = self.coarse_pre, self.coarse_post
                 plan.pre0, plan.post0 = (self.pre_sweeps, self.post_sweeps) if first == 0 else (plan.pre, plan.post)

@@ -66,3 +66,18 @@ def test_sweep_counts_set_on_the_projector(sweeps):
     else:
         assert bool(torch.isfinite(got).all()) and float(got.abs().max()) > 0
     projector.close()
+
+@pytest.mark.parametrize('sweeps', [(0, 4), (3, 0)])
+def test_sweep_counts_set_on_a_collider_projector(sweeps):
+    from tests.test_gpu_graph_resident import build
+    results = []
+    for resident in (True, False):
+        projector, faces = build((32, 32, 32))
+        projector.use_resident = resident
+        projector.pre_sweeps, projector.post_sweeps = sweeps
+        projector.coarse_pre, projector.coarse_post = sweeps
+        out = [torch.zeros_like(f) for f in faces]
+        projector.project(faces, out, 0.02)
+        results.append(projector.pressure.clone())
+        projector.close()
+    assert torch.equal(*results) and bool(results[0].any())
