@@ -64,8 +64,9 @@ class MultigridPressureProjector(PressureProjector):
             inv = neumann_inverse(coarsest, grid.extent)
             self.coarse_matrix = torch.as_tensor(inv, dtype=torch.float64).to(dev.device)
             self.coarse_kernel = KernelHandle('coarse_pressure.glsl')
-            # the same inverse in its separable form, as the cycles apply it
-            self.coarse_basis = torch.as_tensor(neumann_basis(coarsest, grid.extent)).to(dev.device)
+            if not self._separate_passes:
+                # the same inverse in its separable form, as the native cycles apply it
+                self.coarse_basis = torch.as_tensor(neumann_basis(coarsest, grid.extent)).to(dev.device)
         self.pre_sweeps = s.mg_pre_sweeps or 3
         self.post_sweeps = s.mg_post_sweeps or 3
         self._relaxation = None

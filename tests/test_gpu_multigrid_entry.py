@@ -81,3 +81,10 @@ def test_sweep_counts_set_on_a_collider_projector(sweeps):
         results.append(projector.pressure.clone())
         projector.close()
     assert torch.equal(*results) and bool(results[0].any())
+
+
+def test_the_coarse_basis_is_made_for_whole_cycles_only():
+    assert make('FP32', (64, 64, 64)).coarse_basis is not None
+    projector = make('BF16', (64, 64, 64))
+    assert projector.coarse_basis is None and projector.coarse_matrix is not None
+    assert solve(projector, 1)[2] == 1
