@@ -116,7 +116,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         self.speculate = True
         self._pending_refresh = None
         self._alarm = None       # of the resident plans (made with the first)
-        self._loops = {}
+        self._captured = {}      # tolerance solves as captured loops (_device_solve)
         # [cycles of the last solve, cycles of all device-loop solves, decisions]
         self._counters = torch.zeros(3, dtype=torch.int32, device=dev.device)
         self._host_total = 0
@@ -202,7 +202,7 @@ class SolidMultigridProjector(SolidPressureProjector):
         self._coarse_solve()
         self._graphs = {}
         self._pending_refresh = None
-        if getattr(self, '_loops', None):
+        if self._captured:
             torch.cuda.synchronize(dev.device)
             self._free_loops()
         self._tail, self.tail_start = self._make_tail()
@@ -661,7 +661,6 @@ class SolidMultigridProjector(SolidPressureProjector):
                          int(s.pressure_max_cycles), ptr(self._counters), self.device.s)
         self._sweeps_per_cycle = self._cycle_sweeps()
         if tolerance:
-            self._loops['resident'] = (None, *self._resident(0))      # this solve's loop on the device
             self._cycles_on_device = True
         else:
             self.last_cycles = budget
@@ -697,10 +696,10 @@ class SolidMultigridProjector(SolidPressureProjector):
         loop counts outer iterations (see ``_capture_loop``)."""
         dev = self.device
         key = ('refine' if refine else 'loop', self.levels[0]['p'].data_ptr(), self.levels[0]['q'].data_ptr())
-        entry = self._loops.get(key)
+        entry = self._captured.get(key)
         if entry is None:
             entry = self._capture_loop(refine)
-            self._loops[key] = entry
+            self._captured[key] = entry
         handle, per_cycle, calls = entry
         dev.call('ffx_loop_launch', handle, dev.s)
         dev.calls += calls - 1
@@ -806,11 +805,16 @@ class SolidMultigridProjector(SolidPressureProjector):
             dev.calls = saved_calls
         return loop, per_cycle, calls
 
+    @property
+    def _loops(self):
+        """Where tolerance solves loop on the device: the captured loops, and the plan of whole solves."""
+        whole = self._residents.get(0)
+        return self._captured | ({'resident': whole} if whole else {})
+
     def _free_loops(self):
-        for handle, _, _ in self._loops.values():
-            if handle is not None:      # a resident solve's loop is its plan
-                self.device.lib.ffx_loop_destroy(handle)
-        self._loops = {}
+        for handle, _, _ in self._captured.values():
+            self.device.lib.ffx_loop_destroy(handle)
+        self._captured = {}
 
     def gradient_links(self):
         # the link bytes follow the mask (recomputed on every collider move)
@@ -867,7 +871,7 @@ class SolidMultigridProjector(SolidPressureProjector):
             'aggregation': 'connected_children_only'}
 
     def close(self):
-        if getattr(self, '_loops', None):
+        if self._captured:
             torch.cuda.synchronize(self.device.device)
             self._free_loops()
         self._graphs = {}
