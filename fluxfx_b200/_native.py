@@ -345,6 +345,7 @@ _PROTOTYPES = {
     'ffx_batch_create': (C.c_int, [P(FfxBatchDomain), i32, vp, i64, P(vp)]),
     'ffx_batch_set_config': (C.c_int, [vp, i32, i32, i32]),
     'ffx_batch_tune_pass': (C.c_int, [vp, i32, vp]),
+    'ffx_batch_has_pass': (C.c_int, [vp, i32]),
     'ffx_batch_graph': (C.c_int, [vp, i32, P(vp)]),
     'ffx_batch_launch': (C.c_int, [vp, vp, i32, vp]),
     'ffx_batch_graph_free': (C.c_int, [vp]),

@@ -231,7 +231,7 @@ class BatchedSmoke:
     def tune(self, repeats=5, cache=None):
         """Time every (tile shape, persistent grid) of each pass kind alone on
         the plan's buffers and keep the fastest; returns {pass: (shape, grid,
-        ms)}. With ``cache`` (a JSON file) results are reused per device and
+        ms)}, with (0, 0, 0.0) for a pass that this plan's steps do not launch. With ``cache`` (a JSON file) results are reused per device and
         domain shapes."""
         dev = torch.cuda.get_device_name(self.device.device)
         key = f'{dev}|{self.signature()}'
@@ -245,6 +245,9 @@ class BatchedSmoke:
         stream = torch.cuda.ExternalStream(self.stream) if self.stream else torch.cuda.current_stream()
         best = {}
         for kind in TUNABLE:
+            if not self.lib.ffx_batch_has_pass(self.plan, kind):
+                best[N.PASS_NAMES[kind]] = (0, 0, 0.0)
+                continue
             results = []
             for shape in ((0,) if kind in N.FIXED_TILE_PASSES else range(len(SHAPES))):
                 for grid in GRIDS:

@@ -674,7 +674,8 @@ int build(FfxBatchPlan& P, std::vector<char>& host) {
         for (auto* list : {&P.pre[0], &P.post[0], &P.cycle})
             for (auto& L : *list)
                 if (L.kind == kind && (!found || volume(L) > volume(*found))) found = &L;
-        if ((kind == kResidualMax || kind == kL0ResidualMax) && P.resmax.kind == kind) found = &P.resmax;
+        if (P.resident_first != 0 && (kind == kResidualMax || kind == kL0ResidualMax) && P.resmax.kind == kind)
+            found = &P.resmax;
         if (kind == kGradient) {
             P.tune[kind] = B.launch(kGradient, all, [&](int d, char* out, FfxBatchPlan::Entry& e) {
                 const FfxBatchDomain& D = P.dom[d];
@@ -838,6 +839,10 @@ int ffx_batch_set_config(FfxBatchPlan* plan, int32_t kind, int32_t shape, int32_
     plan->shape[kind] = shape;
     plan->grid[kind] = grid;
     return FFX_OK;
+}
+
+int ffx_batch_has_pass(const FfxBatchPlan* plan, int32_t kind) {
+    return plan && kind >= 0 && kind < kBatchKinds && !plan->tune[kind].entries.empty();
 }
 
 int ffx_batch_tune_pass(FfxBatchPlan* plan, int32_t kind, void* stream) {

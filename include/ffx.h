@@ -883,6 +883,9 @@ int ffx_batch_set_config(FfxBatchPlan* plan, int32_t kind, int32_t shape, int32_
  * writes scratch fields that the step recomputes, the gradient pass writes the
  * predictor faces instead of the velocity). */
 int ffx_batch_tune_pass(FfxBatchPlan* plan, int32_t kind, void* stream);
+/* 1 when the plan's steps launch this pass kind (a resident solve has no passes of
+ * its own), else 0: there is nothing to tune. */
+int ffx_batch_has_pass(const FfxBatchPlan* plan, int32_t kind);
 /* Capture `steps` steps (starting from the plan's current parity) into an
  * instantiated CUDA graph with one conditional WHILE node per solve. */
 int ffx_batch_graph(FfxBatchPlan* plan, int32_t steps, void** graph_exec);
