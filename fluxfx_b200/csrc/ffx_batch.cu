@@ -312,15 +312,7 @@ int resident(int kind) {
     return r > 0 ? r : 1;
 }
 
-cudaError_t issue(FfxBatchPlan& P, const FfxBatchPlan::Launch& L, cudaStream_t st) {
-    if (L.kind == kResident) {
-        gres::Call A = {};
-        A.batched = A.aligned = 1;
-        return gres::launch(P.resident_first == 0, reinterpret_cast<const gres::Domain*>(P.ws + P.resident_domains),
-                            P.count, P.resident_blocks, P.resident_smem, A, st) == FFX_OK
-                   ? cudaSuccess
-                   : cudaErrorLaunchFailure;
-    }
+cudaError_t issue_pass(FfxBatchPlan& P, const FfxBatchPlan::Launch& L, cudaStream_t st) {
     if (L.entries.empty()) return cudaSuccess;
     BatchMap M = make_map(P, L);
     if (M.total == 0) return cudaSuccess;
@@ -573,7 +565,7 @@ bool plan_resident(Builder& B, int first) {
         R.max_cycles = D.max_cycles;
         memcpy(B.host.data() + P.resident_domains + d * sizeof R, &R, sizeof R);
         P.resident_blocks += chosen[d].blocks;
-        P.resident_bytes += (int64_t)align_up(8 * gres::words_of(specs[d], dist[d], chosen[d]));
+        P.resident_bytes += (int64_t)align_up(8 * gres::words_of(specs[d], dist[d]));
     }
     return true;
 }
@@ -709,29 +701,35 @@ int build(FfxBatchPlan& P, std::vector<char>& host) {
 
 const StepRule* rules_of(const FfxBatchPlan& P) { return reinterpret_cast<const StepRule*>(P.rules); }
 
-cudaError_t issue_list(FfxBatchPlan& P, const std::vector<FfxBatchPlan::Launch>& list, cudaStream_t st) {
-    for (const auto& L : list) {
-        cudaError_t e = issue(P, L, st);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+// Launches one entry of a plan; a status with its message (the resident solve's own).
+int issue(FfxBatchPlan& P, const FfxBatchPlan::Launch& L, cudaStream_t st, const char* what) {
+    if (L.kind != kResident) return cuda_status(issue_pass(P, L, st), what);
+    gres::Call A = {};
+    A.batched = A.aligned = 1;
+    return gres::launch(P.resident_first == 0, reinterpret_cast<const gres::Domain*>(P.ws + P.resident_domains),
+                        P.count, P.resident_blocks, P.resident_smem, A, st);
+}
+
+int issue_list(FfxBatchPlan& P, const std::vector<FfxBatchPlan::Launch>& list, cudaStream_t st, const char* what) {
+    for (const auto& L : list)
+        if (int rc = issue(P, L, st, what)) return rc;
+    return FFX_OK;
 }
 
 // One step captured on `st` (capturing) with the solve loop as a WHILE node
 // whose body is captured on `side`.
 int capture_step(FfxBatchPlan& P, int par, cudaStream_t st, cudaStream_t side) {
-    cudaError_t e = issue_list(P, P.pre[par], st);
-    if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: passes before the solve");
+    int rc = issue_list(P, P.pre[par], st, "ffx_batch_graph: passes before the solve");
+    if (rc) return rc;
     if (P.resident_first == 0) {
         FfxBatchPlan::Launch L;
         L.kind = kResident;
-        e = issue(P, L, st);
-        if (e == cudaSuccess) {
-            batch_count_kernel<<<1, 32, 0, st>>>(P.state, P.count, P.guard);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = issue_list(P, P.post[par], st);
-        if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: resident solve");
+        rc = issue(P, L, st, "ffx_batch_graph: resident solve");
+        if (rc) return rc;
+        batch_count_kernel<<<1, 32, 0, st>>>(P.state, P.count, P.guard);
+        rc = cuda_status(cudaGetLastError(), "ffx_batch_graph: cycle count");
+        if (!rc) rc = issue_list(P, P.post[par], st, "ffx_batch_graph: passes after the solve");
+        if (rc) return rc;
         batch_step_end_kernel<<<1, 64, 0, st>>>(P.state, rules_of(P), P.solve, P.count, P.guard);
         return cuda_status(cudaGetLastError(), "ffx_batch_graph: step end");
     }
@@ -739,7 +737,7 @@ int capture_step(FfxBatchPlan& P, int par, cudaStream_t st, cudaStream_t side) {
     cudaGraph_t graph = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     size_t ndeps = 0;
-    e = cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &ndeps);
+    cudaError_t e = cudaStreamGetCaptureInfo(st, &status, nullptr, &graph, &deps, &ndeps);
     if (e != cudaSuccess || status != cudaStreamCaptureStatusActive)
         return cuda_status(e != cudaSuccess ? e : cudaErrorStreamCaptureInvalidated, "ffx_batch_graph: capture info");
     cudaGraphConditionalHandle handle;
@@ -755,20 +753,20 @@ int capture_step(FfxBatchPlan& P, int par, cudaStream_t st, cudaStream_t side) {
     cudaGraph_t body = params.conditional.phGraph_out[0];
     e = cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: body capture");
-    cudaError_t eb = issue(P, P.resmax, side);
-    if (eb == cudaSuccess) {
+    rc = issue(P, P.resmax, side, "ffx_batch_graph: solve body");
+    if (!rc) {
         batch_decide_kernel<<<1, 64, 0, side>>>(P.state, P.solve, P.count, P.guard, handle);
-        eb = cudaGetLastError();
+        rc = cuda_status(cudaGetLastError(), "ffx_batch_graph: solve body");
     }
-    if (eb == cudaSuccess) eb = issue_list(P, P.cycle, side);
+    if (!rc) rc = issue_list(P, P.cycle, side, "ffx_batch_graph: solve body");
     cudaGraph_t captured = nullptr;
     e = cudaStreamEndCapture(side, &captured);
-    if (eb != cudaSuccess) return cuda_status(eb, "ffx_batch_graph: solve body");
+    if (rc) return rc;
     if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: end of body capture");
     e = cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies);
     if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: capture dependencies");
-    e = issue_list(P, P.post[par], st);
-    if (e != cudaSuccess) return cuda_status(e, "ffx_batch_graph: passes after the solve");
+    rc = issue_list(P, P.post[par], st, "ffx_batch_graph: passes after the solve");
+    if (rc) return rc;
     batch_step_end_kernel<<<1, 64, 0, st>>>(P.state, rules_of(P), P.solve, P.count, P.guard);
     return cuda_status(cudaGetLastError(), "ffx_batch_graph: step end");
 }
@@ -848,7 +846,7 @@ int ffx_batch_has_pass(const FfxBatchPlan* plan, int32_t kind) {
 int ffx_batch_tune_pass(FfxBatchPlan* plan, int32_t kind, void* stream) {
     FFX_REQUIRE(plan && kind >= 0 && kind < kBatchKinds, "ffx_batch_tune_pass: invalid arguments");
     cudaStream_t st = as_stream(stream);
-    int e = cuda_status(issue(*plan, plan->tune[kind], st), "ffx_batch_tune_pass");
+    int e = issue(*plan, plan->tune[kind], st, "ffx_batch_tune_pass");
     if (e) return e;
     if (kind == kScaleZero || kind == kGradient || kind == kResidualMax || kind == kL0ResidualMax) {
         batch_clear_kernel<<<1, 64, 0, st>>>(plan->state, plan->count);

@@ -30,7 +30,7 @@ struct Candidate {
 // SMs at once; false when they do not fit. dist: levels in tiles, per domain.
 bool plan_blocks(const Spec* specs, int count, int sms, std::vector<Candidate>& chosen, std::vector<int>& dist);
 // 64-bit words of a domain's published rows and header.
-int64_t words_of(const Spec& S, int dist, const Candidate& c);
+int64_t words_of(const Spec& S, int dist);
 // The domain's record; returns the bytes of shared memory its blocks need.
 int fill(const Spec& S, int dist, const Candidate& c, int first_block, u64* ws, Domain& D);
 int launch(bool links, const Domain* domains, int count, int blocks, int smem, const Call& A, cudaStream_t st);

@@ -108,11 +108,10 @@ bool plan_blocks(const Spec* specs, int count, int sms, std::vector<Candidate>& 
     }
 }
 
-int64_t words_of(const Spec& S, int dist, const Candidate& c) {
+int64_t words_of(const Spec& S, int dist) {
     int64_t words = 2 * kMaxTiles + 2 + kHeader;
     for (int k = 0; k < dist; ++k) words += 2 * 4 * slots_of(S.level[k]);
     if (dist < S.count) words += 2 * 4 * slots_of(S.level[dist]);
-    (void)c;
     return words;
 }
 
@@ -297,7 +296,7 @@ int ffx_graph_plan(FfxGraphPlan* P) {
     P->tile[0] = c[0].ty;
     P->tile[1] = c[0].tz;
     P->tail = dist[0];
-    P->workspace_bytes = kDomainBytes + 8 * gres::words_of(S, dist[0], c[0]);
+    P->workspace_bytes = kDomainBytes + 8 * gres::words_of(S, dist[0]);
     return FFX_OK;
 }
 
