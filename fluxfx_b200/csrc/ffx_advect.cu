@@ -167,8 +167,9 @@ __device__ __forceinline__ void face_predictor_axis(const PredParams<T>& P, Face
     F3 p = {((float)f.x + ox) * d.h[0], ((float)f.y + oy) * d.h[1], ((float)f.z + oz) * d.h[2]};
     F3 v0 = start_velocity_face<EXACT<T, MASK>, P2>(d, smp, p, f.axis, f.x, f.y, f.z);
     F3 dep = backtrace_s<MASK, EXACT<T, MASK>, P2>(d, smp, solid, halo, p, v0, dt, cv);
-    float value = smp.template sample<EXACT<T, MASK>>(f.axis, cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - ox, cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - oy,
-                             cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - oz);
+    float value = smp.template sample<EXACT<T, MASK>>(f.axis, cells<EXACT<T, MASK>, P2>(d, dep.x, 0) - ox,
+                                                      cells<EXACT<T, MASK>, P2>(d, dep.y, 1) - oy,
+                                                      cells<EXACT<T, MASK>, P2>(d, dep.z, 2) - oz);
     Store<T>::st(out, f.i, value);
     if (float* D = P.dep[f.axis]) {
         const int nf = P.nf[f.axis];
@@ -291,8 +292,10 @@ __device__ __forceinline__ void advect_velocity_axis(const VelParams<T>& P, Face
                         arr.y > hib[1] || arr.z > hib[2]);
             if (MASK && ok) ok = safe_correction_from<P2>(d, P.solid, P.halo, cv, p, dep, mid2, arr);
             if (ok) {
-                float pa = smp.template sample<EXACT<T, MASK>>(3 + axis, cells<EXACT<T, MASK>, P2>(d, arr.x, 0) - off[0], cells<EXACT<T, MASK>, P2>(d, arr.y, 1) - off[1],
-                                      cells<EXACT<T, MASK>, P2>(d, arr.z, 2) - off[2]);
+                float pa = smp.template sample<EXACT<T, MASK>>(3 + axis,
+                                                               cells<EXACT<T, MASK>, P2>(d, arr.x, 0) - off[0],
+                                                               cells<EXACT<T, MASK>, P2>(d, arr.y, 1) - off[1],
+                                                               cells<EXACT<T, MASK>, P2>(d, arr.z, 2) - off[2]);
                 float val = Store<T>::ld(pred, f.i) + 0.5f * (Store<T>::ld(orig, f.i) - pa);
                 // min / max of the 8 corners around the departure point, clamped to the grid
                 float lo, hi;
@@ -1517,27 +1520,31 @@ size_t scalar_final_desc(const FfxBatchDomain& D, int parity, void* out) {
     return sizeof(ScalarFinal<float>);
 }
 
-cudaError_t face_predictor(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    (M.pow2 ? batch_predictor_kernel<true> : batch_predictor_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const PredParams<float>*)descs, state);
+// The kernel's form for power-of-two grids where all of the launch's are, else the general one.
+template <class Desc, class... Args>
+cudaError_t launch_batch(void (*pow2)(BatchMap, const Desc*, const BatchState*, Args...),
+                         void (*general)(BatchMap, const Desc*, const BatchState*, Args...), const BatchMap& M,
+                         const void* descs, BatchState* state, int grid, cudaStream_t st, Args... args) {
+    (M.pow2 ? pow2 : general)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const Desc*)descs, state, args...);
     return cudaGetLastError();
 }
+
+cudaError_t face_predictor(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
+    return launch_batch(batch_predictor_kernel<true>, batch_predictor_kernel<false>, M, descs, state, grid, st);
+}
 cudaError_t advect_velocity(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    (M.pow2 ? batch_velocity_kernel<true> : batch_velocity_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const VelParams<float>*)descs, state);
-    return cudaGetLastError();
+    return launch_batch(batch_velocity_kernel<true>, batch_velocity_kernel<false>, M, descs, state, grid, st);
 }
 cudaError_t scalar_transport(const BatchMap& M, const void* descs, BatchState* state, int reverse, int grid,
                              cudaStream_t st) {
     if (reverse)
-        (M.pow2 ? batch_scalar_reverse_kernel<true> : batch_scalar_reverse_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarXport<float>*)descs,
-                                                                               state);
-    else
-        (M.pow2 ? batch_scalar_transport_kernel<true> : batch_scalar_transport_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(
-            M, (const ScalarXport<float>*)descs, state, 1.f);
-    return cudaGetLastError();
+        return launch_batch(batch_scalar_reverse_kernel<true>, batch_scalar_reverse_kernel<false>, M, descs, state,
+                            grid, st);
+    return launch_batch(batch_scalar_transport_kernel<true>, batch_scalar_transport_kernel<false>, M, descs, state,
+                        grid, st, 1.f);
 }
 cudaError_t advect_scalars(const BatchMap& M, const void* descs, BatchState* state, int grid, cudaStream_t st) {
-    (M.pow2 ? batch_scalars_kernel<true> : batch_scalars_kernel<false>)<<<grid_of(M, grid), kBatchThreads, 0, st>>>(M, (const ScalarFinal<float>*)descs, state);
-    return cudaGetLastError();
+    return launch_batch(batch_scalars_kernel<true>, batch_scalars_kernel<false>, M, descs, state, grid, st);
 }
 
 int advect_resident_blocks(int kind) {
