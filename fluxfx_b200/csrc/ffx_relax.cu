@@ -122,6 +122,7 @@ __device__ __forceinline__ void sweep(const Box& b, const Lane& l, const Weights
         c = P[i];
     }
     const float wx = b.w[0], wy = b.w[1], wz = b.w[2];
+    const int in_row = b.n[0] - (b.gx + 4 * l.x);
     for (int z = z0; z < z1; ++z, i += plane) {
         const float4 r = R[i];
         float4 k = W.k, d = W.d;
@@ -146,7 +147,7 @@ __device__ __forceinline__ void sweep(const Box& b, const Lane& l, const Weights
             lo = c;
             c = hi;
         }
-        Q[i] = weighted(k, out);
+        Q[i] = weighted<MASK>(k, in_row, out);
     }
 }
 

@@ -95,9 +95,14 @@ __device__ __forceinline__ void weights_of(unsigned codes, const float2* kd, flo
 
 // A sweep's result: 0 in the cells without a weight (colliders, isolated cells,
 // padding), whatever stands beside them. Selected, not multiplied: 0 times an
-// infinity would carry it through a wall.
-__device__ __forceinline__ float4 weighted(float4 k, float4 o) {
-    return make_float4(k.x > 0.f ? o.x : 0.f, k.y > 0.f ? o.y : 0.f, k.z > 0.f ? o.z : 0.f, k.w > 0.f ? o.w : 0.f);
+// infinity would carry it through a wall. Without colliders only a row's padding
+// has none: `left` cells of the float4 lie in the row (testing the weights there
+// too took 128^3 from 218 to 224 us per projection).
+template <bool MASK>
+__device__ __forceinline__ float4 weighted(float4 k, int left, float4 o) {
+    if (MASK)
+        return make_float4(k.x > 0.f ? o.x : 0.f, k.y > 0.f ? o.y : 0.f, k.z > 0.f ? o.z : 0.f, k.w > 0.f ? o.w : 0.f);
+    return make_float4(o.x, left > 1 ? o.y : 0.f, left > 2 ? o.z : 0.f, left > 3 ? o.w : 0.f);
 }
 
 // n / d for 0 <= n < 2^16 and 1 <= d < 2^12, with inv = 1 / d: (n + 1/2) / d is
@@ -296,6 +301,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
     const int out_step = 4 * v.x4 * v.n[1];
     const int64_t copy = 4 * (int64_t)v.x4 * v.n[1] * v.n[2];
     const float wx = v.w[0], wy = v.w[1], wz = v.w[2];
+    const int in_row = v.n[0] - 4 * x;
     const bool left = x > 0, right = x + 1 < v.x4, rim_y = y == 0 || y == v.ty - 1;
     auto formed = [&](const float4* P, int j, bool blank, float4& lo, float4& c, float4 hi) {
         const int i = i0 + j * v.plane;
@@ -307,7 +313,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             const int gz = v.z0 + z0 + j;
             if (gz == 0 || gz == v.n[2] - 1) weights_of(edge, kd, k, d);
         }
-        if (blank) return weighted(k, make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w));
+        if (blank) return weighted<MASK>(k, in_row, make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w));
         const float4 ym = P[i - v.x4], yp = P[i + v.x4];
         const float* row = reinterpret_cast<const float*>(P) + 4 * i;
         const float xl = left ? row[-1] : 0.f, xr = right ? row[4] : 0.f;
@@ -320,7 +326,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
                         fmaf(k.z, fmaf(-d.z, c.z, o.z), c.z), fmaf(k.w, fmaf(-d.w, c.w, o.w), c.w));
         lo = c;
         c = hi;
-        return weighted(k, o);
+        return weighted<MASK>(k, in_row, o);
     };
     for (int s = 0; s < count; ++s) {
         const bool blank = zero && s == 0;
