@@ -29,9 +29,10 @@ class PressureProjector:
         self._field_dtype = torch.bfloat16 if self.settings.storage == 'BF16' else torch.float32
         self._storage = N.FFX_F32 if self._field_dtype == torch.float32 else N.FFX_BF16
         self._mask = getattr(self.device, 'mask', None)
-        # 16-bit storage keeps a launch per pass: the whole-solve kernels round their
-        # sums in another order, and a pressure whose last bit differs flips stored
-        # 16-bit velocities, which the next step's divergence shows (1e-4 of its pressure)
+        # 16-bit storage keeps a launch per pass: the whole-solve kernels have no form
+        # that rounds in the passes' order, and a pressure whose last bit differs flips
+        # stored 16-bit velocities, which the next step's divergence shows (1e-4 of its
+        # pressure)
         self._separate_passes = self._storage == N.FFX_BF16
         self._jacobi = None       # the Jacobi solve's plan (made on first use)
         self._classes = None      # open-neighbour codes of the mask (ffx_relax_classes)

@@ -219,11 +219,11 @@ __device__ __forceinline__ float dot3(const F3& a, const F3& b) { return (a.x * 
 //    rounded constant and one product, the two roundings of p n / e, at a tenth
 //    of its instructions), and start points at cell and face centres at their
 //    exact half-integer coordinates.
-// The passes are bound by instruction issue (75-87 % of the slots; DRAM under
-// 17 %), so instructions are what a sample costs. Measured, all transport passes
+// The passes are bound by instruction issue (80-83 % of the slots, 57 % in the final
+// scalar pass; DRAM under 20 %), so instructions are what a sample costs. Measured, all transport passes
 // of a step, clamped corners one by one and weighted sums everywhere -> this:
 // 128 x 96 x 112 FP32 without colliders 455 -> 328 us; with colliders, 256^3 BF16
-// 4.8 -> 4.1 ms and 96 x 80 x 112 FP32 470 -> 446 us.
+// 4.8 -> 4.4 ms and 96 x 80 x 112 FP32 470 -> 446 us.
 
 // (1 - t) a + t b: exactly a at t = 0 and b at t = 1, for finite a and b.
 __device__ __forceinline__ float lerp(float a, float b, float t) { return fmaf(t, b, fmaf(-t, a, a)); }

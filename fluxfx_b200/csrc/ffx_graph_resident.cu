@@ -71,7 +71,10 @@ bool candidates(const Spec& S, int sms, std::vector<Candidate>& out, int& dist) 
                 x4 * (2 * (ty + tz) + 4) > kThreads * kRimItems || x4 * (ty + 2) >= 4096 ||
                 16 * tile_f4(S, dist, ty, tz, false) > resident::kSmem)
                 continue;
-            // a sweep's work per block: its cells, and its rim's words and addresses
+            // a sweep's work per block: its cells, and its rim's words and addresses. Of all
+            // tiles that fit, the least cost was the fastest at 32^3, 64 x 32 x 64, 48 x 96 x
+            // 48, 64^3, 96 x 80 x 112 and 96 x 96 x 160 (two V(4,4) cycles: 85 us at 32^3 with
+            // the chosen tile, 222 with the worst; 352 and 516 at 96 x 80 x 112)
             out.push_back(Candidate{ty, tz, tiles + (tail ? 1 : 0), 1.0 * x4 * ty * tz + 0.6 * x4 * (2 * (ty + tz) + 4)});
         }
     return !out.empty();

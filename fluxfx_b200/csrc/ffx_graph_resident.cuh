@@ -17,10 +17,11 @@
 //
 // Measured, a step with a sphere and a box, separate passes -> resident:
 // 96 x 80 x 112 (two V(4,4) cycles) 783 -> 716 us, 96 x 96 x 160 (five) 2226 ->
-// 1838 us. A cycle of 96 x 96 x 160 takes 129 us. What bounds it: a sweep of a
-// level whose runs are one float4 is 1000 cycles of latency (loads 250, sums and
-// quotient 400, publishing 200) and 1400 of exchange; packed FP32 instructions
-// (f32x2) changed nothing, so neither issue nor bandwidth does.
+// 1838 us. A cycle of 96 x 96 x 160 takes 129 us. What bounds it is the latency of
+// a sweep and of its exchange: a quarter of the issue slots are used, and a warp
+// waits 8 cycles at block barriers (behind the warps that poll) and 2 for loads per
+// instruction it issues (profiles/resident_solves.txt); packed FP32 instructions
+// (f32x2) changed nothing.
 #pragma once
 #include "ffx_batch.cuh"
 #include "ffx_resident.cuh"

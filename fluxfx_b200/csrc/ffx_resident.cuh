@@ -18,11 +18,13 @@
 //                           residual and publishes the correction.
 // With dist = 0 one block holds every level and reads and writes global memory.
 //
-// What bounds a sweep now is the exchange: 1.2 us at 32^3, where a block
-// relaxes 64 float4, of which the words' way through the L2 is about half.
+// What bounds a sweep now is the exchange and the latency of a few instructions:
+// 1.2 us at 32^3, where a block relaxes 64 float4; a third of the issue slots are
+// used, and the warps wait at barriers, behind those that poll
+// (profiles/resident_solves.txt).
 // Measured, us per sweep, a launch per sweep (T fused sweeps per launch) ->
-// resident: 75 x 61 x 93 5.5 (3.5) -> 2.0, 64^3 4.1 (3.4) -> 1.6, 127^3 12 (11)
-// -> 4.8; us per V(3,3) cycle: 128^3 250 (143) -> 73, 32^3 95 (40) -> 24.
+// resident: 75 x 61 x 93 5.5 (3.5) -> 2.1, 64^3 4.1 (3.4) -> 1.5, 127^3 12 (11)
+// -> 5.3; us per V(3,3) cycle: 128^3 250 (143) -> 73, 32^3 95 (40) -> 24.
 //
 // Blocks wait for one another, so the launch is cooperative (all blocks
 // resident at once); every wait is bounded: after kSpinLimit polls a block
