@@ -70,6 +70,8 @@ class MultigridPressureProjector(PressureProjector):
         self.pre_sweeps = s.mg_pre_sweeps or 3
         self.post_sweeps = s.mg_post_sweeps or 3
         self._relaxation = None
+        if len(shapes) == 1:
+            self._make_jacobi()
         self._whole_cycles()
         self.last_cycles = 0
         self.last_coarse_solves = 0

@@ -34,7 +34,7 @@ class PressureProjector:
         # stored 16-bit velocities, which the next step's divergence shows (1e-4 of its
         # pressure)
         self._separate_passes = self._storage == N.FFX_BF16
-        self._jacobi = None       # the Jacobi solve's plan (made on first use)
+        self._jacobi = None       # the Jacobi solve's plan
         self._classes = None      # open-neighbour codes of the mask (ffx_relax_classes)
         self._solids = solids_struct(self.device)
         self.wall = KernelHandle('pressure_walls.glsl')
@@ -62,6 +62,8 @@ class PressureProjector:
         self.ready = False
         self.last_dt = None
         self.last_iterations = 0
+        if type(self).solve_pressure is PressureProjector.solve_pressure:
+            self._make_jacobi()       # (others make it when they fall back to it)
 
     # -------------------------------------------------------------- helpers
     @property
@@ -236,6 +238,19 @@ class PressureProjector:
     def _starts_from_zero(self, dt, previous_dt):
         return previous_dt != dt
 
+    def _make_jacobi(self):
+        """The whole Jacobi solve's plan and workspace (not for separate passes). Made
+        before the first solve, which may be under capture: what a capture zeroes is
+        zero in its replays only."""
+        if self._jacobi is not None or self._separate_passes:
+            return
+        if self._mask is not None:
+            nx, ny, nz = self.grid.shape
+            with self.device.ordered():
+                self._classes = torch.empty((nz, ny, (nx + 3) // 4 * 4), dtype=torch.uint8, device=self.device.device)
+        self._jacobi = Relaxation(self.device, [self.grid.shape], self.grid.extent, self.settings.pressure_relaxation,
+                                  last=4096, classes=self._classes)
+
     def solve_pressure(self, dt, previous_dt):
         # Jacobi smooths across cells: scale the work with resolution squared.
         scaled = ceil(self.settings.pressure_iterations * max(1.0, (max(self.grid.shape) / 64) ** 2))
@@ -250,14 +265,7 @@ class PressureProjector:
                                  ptr(self.before), dt, omega, ptr(self.spare), self.device.s)
                 self.pressure, self.spare = self.spare, self.pressure
             return
-        if self._jacobi is None:
-            if self._mask is not None:
-                nx, ny, nz = self.grid.shape
-                with self.device.ordered():
-                    self._classes = torch.empty((nz, ny, (nx + 3) // 4 * 4), dtype=torch.uint8,
-                                                device=self.device.device)
-            self._jacobi = Relaxation(self.device, [self.grid.shape], self.grid.extent,
-                                      self.settings.pressure_relaxation, last=4096, classes=self._classes)
+        self._make_jacobi()
         if self._classes is not None:
             # the mask may have moved since the last solve
             self.device.call('ffx_relax_classes', self._n3, self._mask_ptr(), ptr(self._classes), self.device.s)

@@ -123,6 +123,8 @@ class SolidMultigridProjector(SolidPressureProjector):
         self._sweeps_per_cycle = 0
         self._cycle_factor = s.ir_inner_cycles if s.pressure_method == 'IR' else 1
         self._build_hierarchy()
+        if len(self.levels) == 1:
+            self._make_jacobi()
         self._rmax = torch.zeros(2, dtype=torch.float32, device=dev.device)
 
     # The cycle count of the last solve lives on the device after a device-loop
