@@ -7,6 +7,7 @@ the chip; larger ones several sweeps per launch.
 """
 import ctypes as C
 import itertools
+import threading
 
 import torch
 
@@ -15,6 +16,7 @@ from .. import _native as N
 
 _WORDS = 4096
 _page = None
+_lock = threading.Lock()
 _taken = itertools.count()
 
 
@@ -29,8 +31,9 @@ class Alarm:
 
     def __init__(self):
         global _page
-        if _page is None:
-            _page = torch.zeros(_WORDS, dtype=torch.int32, pin_memory=True)
+        with _lock:
+            if _page is None:
+                _page = torch.zeros(_WORDS, dtype=torch.int32, pin_memory=True)
         self.address = _page.data_ptr() + 4 * (next(_taken) % _WORDS)
         self._view = C.c_int32.from_address(self.address)
 
