@@ -147,7 +147,7 @@ __device__ __forceinline__ void sweep(const Box& b, const Lane& l, const Weights
             lo = c;
             c = hi;
         }
-        Q[i] = weighted<MASK>(k, in_row, out);
+        Q[i] = weighted<MASK, true>(k, in_row, out);
     }
 }
 
@@ -682,10 +682,10 @@ int tail_bytes(const FfxRelaxPlan& P, int first) {
     return 16 * tail_f4(P, first) + (P.basis ? 16 * cells_of(P.level[P.count - 1].grid.n) : 0);
 }
 
-template <bool MASK, bool ONE>
+template <bool MASK, bool ONE, bool RAGGED>
 int launch_resident(const Params& A, int blocks, int smem, cudaStream_t st) {
     static std::atomic<uint64_t> ready{0};
-    auto kernel = resident::resident_kernel<MASK, ONE>;
+    auto kernel = resident::resident_kernel<MASK, ONE, RAGGED>;
     if (int s = allow_smem(kernel, ready)) return s;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
@@ -717,6 +717,13 @@ Params common_params(const FfxRelaxPlan& P, int cycles, float dt) {
     return A;
 }
 
+// Whether rows of the levels from `first` on end in padding.
+bool ragged(const FfxRelaxPlan& P, int first) {
+    for (int k = first; k < P.count; ++k)
+        if (P.level[k].grid.n[0] % 4) return true;
+    return false;
+}
+
 // The levels from `first` on in one block, from zero unless p_in.
 int run_one_block(const FfxRelaxPlan& P, int first, int cycles, float dt, const float* p_in, const float* rhs,
                   float* p_out, cudaStream_t st) {
@@ -729,7 +736,8 @@ int run_one_block(const FfxRelaxPlan& P, int first, int cycles, float dt, const 
     tail_layout(P, first, first, A);
     const int smem = tail_bytes(P, first);
     FFX_REQUIRE(smem <= resident::kSmem && tail_level(P.level[first].grid.n), "relaxation tail out of range");
-    return launch_resident<false, false>(A, 1, smem, st);
+    return ragged(P, first) ? launch_resident<false, false, true>(A, 1, smem, st)
+                            : launch_resident<false, false, false>(A, 1, smem, st);
 }
 
 // The whole solve in one cooperative launch.
@@ -789,10 +797,12 @@ int run_resident(const FfxRelaxPlan& P, int cycles, float dt, bool from_zero, fl
     }
     FFX_REQUIRE(smem <= resident::kSmem, "resident tile out of range");
     const int blocks = A.gy * A.gz + (tail ? 1 : 0);
-    if (P.classes) return one ? launch_resident<true, true>(A, blocks, smem, st)
-                              : launch_resident<true, false>(A, blocks, smem, st);
-    return one ? launch_resident<false, true>(A, blocks, smem, st)
-               : launch_resident<false, false>(A, blocks, smem, st);
+    if (P.classes) return one ? launch_resident<true, true, false>(A, blocks, smem, st)
+                              : launch_resident<true, false, false>(A, blocks, smem, st);
+    if (ragged(P, 0)) return one ? launch_resident<false, true, true>(A, blocks, smem, st)
+                                 : launch_resident<false, false, true>(A, blocks, smem, st);
+    return one ? launch_resident<false, true, false>(A, blocks, smem, st)
+               : launch_resident<false, false, false>(A, blocks, smem, st);
 }
 
 }  // namespace

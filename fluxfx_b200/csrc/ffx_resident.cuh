@@ -98,12 +98,14 @@ __device__ __forceinline__ void weights_of(unsigned codes, const float2* kd, flo
 // A sweep's result: 0 in the cells without a weight (colliders, isolated cells,
 // padding), whatever stands beside them. Selected, not multiplied: 0 times an
 // infinity would carry it through a wall. Without colliders only a row's padding
-// has none: `left` cells of the float4 lie in the row (testing the weights there
-// too took 128^3 from 218 to 224 us per projection).
-template <bool MASK>
+// has none (`left` cells of the float4 lie in the row), and rows of whole float4
+// have no padding (RAGGED false): a projection of 128^3 takes 224 us with the
+// weights tested, 223 with the row's end tested, 219 with neither.
+template <bool MASK, bool RAGGED>
 __device__ __forceinline__ float4 weighted(float4 k, int left, float4 o) {
     if (MASK)
         return make_float4(k.x > 0.f ? o.x : 0.f, k.y > 0.f ? o.y : 0.f, k.z > 0.f ? o.z : 0.f, k.w > 0.f ? o.w : 0.f);
+    if (!RAGGED) return o;
     return make_float4(o.x, left > 1 ? o.y : 0.f, left > 2 ? o.z : 0.f, left > 3 ? o.w : 0.f);
 }
 
@@ -271,7 +273,7 @@ __device__ __forceinline__ void rim_items(const View& v, int (&from)[kRimItems],
 // change places (the caller flips the level by count's parity); with one copy
 // (ONE) it works in place.
 // With an exchange, the rim is current again after every sweep.
-template <bool MASK, bool ONE>
+template <bool MASK, bool ONE, bool RAGGED>
 __device__ __forceinline__ void relax(View& v, int level, const float2* kd, const unsigned* cls, bool zero, int count,
                                       Exchange& ex) {
     const int tid = threadIdx.x;
@@ -315,7 +317,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
             const int gz = v.z0 + z0 + j;
             if (gz == 0 || gz == v.n[2] - 1) weights_of(edge, kd, k, d);
         }
-        if (blank) return weighted<MASK>(k, in_row, make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w));
+        if (blank) return weighted<MASK, RAGGED>(k, in_row, make_float4(k.x * r.x, k.y * r.y, k.z * r.z, k.w * r.w));
         const float4 ym = P[i - v.x4], yp = P[i + v.x4];
         const float* row = reinterpret_cast<const float*>(P) + 4 * i;
         const float xl = left ? row[-1] : 0.f, xr = right ? row[4] : 0.f;
@@ -328,7 +330,7 @@ __device__ __forceinline__ void relax(View& v, int level, const float2* kd, cons
                         fmaf(k.z, fmaf(-d.z, c.z, o.z), c.z), fmaf(k.w, fmaf(-d.w, c.w, o.w), c.w));
         lo = c;
         c = hi;
-        return weighted<MASK>(k, in_row, o);
+        return weighted<MASK, RAGGED>(k, in_row, o);
     };
     for (int s = 0; s < count; ++s) {
         const bool blank = zero && s == 0;
@@ -496,6 +498,7 @@ __device__ __forceinline__ void separable_solve(const View& v, double* wk, const
 
 // ------------------------------------------------------------------- roles
 // A block with whole levels (the tail, or everything when dist = 0).
+template <bool RAGGED>
 __device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (*kd)[28], const Waits& waits,
                                          unsigned base) {
     const int tid = threadIdx.x;
@@ -503,7 +506,7 @@ __device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (
     unsigned flip = 0;       // bit k: level k's pressure is in its second copy
     auto view = [&](int k) { return make_view(A.tv[k], 0, 0, smem, nullptr, flip >> k & 1u); };
     auto smooth = [&](View& v, int k, bool zero, int count) {
-        relax<false, false>(v, 0, kd[k], nullptr, zero, count, none);
+        relax<false, false, RAGGED>(v, 0, kd[k], nullptr, zero, count, none);
         flip ^= (unsigned)(count & 1) << k;
     };
     const int first = A.dist, last = A.count - 1;
@@ -579,7 +582,7 @@ __device__ __forceinline__ void run_tail(const Params& A, float4* smem, float2 (
 }
 
 // A block with a tile of the levels 0 .. dist - 1.
-template <bool MASK, bool ONE>
+template <bool MASK, bool ONE, bool RAGGED>
 __device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (*kd)[28], const Waits& waits,
                                          unsigned base) {
     const int tid = threadIdx.x;
@@ -590,10 +593,10 @@ __device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (
     unsigned* cls = reinterpret_cast<unsigned*>(smem + A.cls_off);
     auto smooth = [&](View& v, int k, bool zero, int count) {
         if (k == 0) {
-            relax<MASK, ONE>(v, 0, kd[0], cls, zero, count, ex);
+            relax<MASK, ONE, RAGGED>(v, 0, kd[0], cls, zero, count, ex);
             if (!ONE) flip ^= (unsigned)(count & 1);
         } else {
-            relax<false, false>(v, k, kd[k], nullptr, zero, count, ex);
+            relax<false, false, RAGGED>(v, k, kd[k], nullptr, zero, count, ex);
             flip ^= (unsigned)(count & 1) << k;
         }
     };
@@ -721,7 +724,8 @@ __device__ __forceinline__ void run_tile(const Params& A, float4* smem, float2 (
     }
 }
 
-template <bool MASK, bool ONE>
+// RAGGED: some level's rows are no multiple of four (any, with a mask: its classes tell).
+template <bool MASK, bool ONE, bool RAGGED>
 __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_constant__ Params A) {
     extern __shared__ float4 smem[];
     __shared__ float2 kd[kLevels][28];
@@ -738,8 +742,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(const __grid_cons
     __syncthreads();
     const unsigned base = A.dist ? A.epochs[blockIdx.x] : 0u;
     const Waits waits = {&dead, A.timeouts, A.alarm};
-    if (tail) run_tail(A, smem, kd, waits, base);
-    else run_tile<MASK, ONE>(A, smem, kd, waits, base);
+    if (tail) run_tail<RAGGED>(A, smem, kd, waits, base);
+    else run_tile<MASK, ONE, RAGGED>(A, smem, kd, waits, base);
     __syncthreads();
     if (tid == 0 && A.dist) A.epochs[blockIdx.x] = base + A.epochs_used;
 }

@@ -73,3 +73,27 @@ def test_non_finite_values_stay_where_single_sweeps_keep_them(shape, walled, fro
     assert np.abs(got[keep] - want[keep]).max() <= bound
     if walled:
         assert not got[solid].any() and np.isfinite(got[:nz // 2, ny // 2:]).all()
+
+
+@pytest.mark.parametrize('shape', [(32, 32, 32), (30, 32, 32), (28, 24, 40), (128, 96, 112)])
+def test_whole_cycles_beside_padding(shape):
+    """A V-cycle's smoothing on a level whose rows end in padding (level 0, or a coarse
+    one below whole float4): what is not finite stays off the cells that no sweep,
+    transfer or coarse solve has carried it to, which with a direct or 80-sweep coarsest
+    level are none, so every cell becomes NaN or infinite, and a clean right-hand side
+    gives a finite pressure in the next solve of the same workspace."""
+    import torch
+    from fluxfx_b200.backend.device import CudaDevice
+    from fluxfx_b200.backend.multigrid import hierarchy_shapes
+    from fluxfx_b200.backend.relax import Relaxation
+    r = Relaxation(CudaDevice(), hierarchy_shapes(shape), tuple(n / max(shape) for n in shape), 2 / 3, pre=3, post=3,
+                   last=80)
+    g = torch.Generator(device='cuda').manual_seed(1)
+    f = torch.randn(shape[::-1], generator=g, device='cuda')
+    p, q = torch.zeros_like(f), torch.zeros_like(f)
+    want = r.run(p, q, f, 2, 1.0, True)[0].clone()
+    bad = f.clone()
+    bad[shape[2] // 2, 1, shape[0] - 1] = float('nan')
+    assert not bool(torch.isfinite(r.run(p, q, bad, 1, 1.0, True)[0]).any())
+    assert torch.equal(r.run(p, q, f, 2, 1.0, True)[0], want) and bool(torch.isfinite(want).all())
+    assert r.timeouts() == 0
